@@ -51,23 +51,22 @@ struct TravStats {
 // Tri.hpp:38-68 bit for bit: the epsilon is (float)0.0000001, 1.0/det is a
 // double division rounded to float, which equals the IEEE float reciprocal
 // (double rounding is innocuous for division when 53 >= 2*24+2).  NaNs pass
-// the range checks exactly as they do in the reference.
+// the range checks exactly as they do in the reference.  The checks are
+// taken together at the end, without the reference's early returns: the
+// lanes of a warp test different triangles, so some lane always needs the
+// rest and every return only splits the warp.
 __device__ __forceinline__ bool mt_hit(f3 v0, f3 v1, f3 v2, f3 o, f3 d, float& t, float& u, float& v) {
   const float EPS = 1.00000001e-07f;
   f3 e1 = xsub(v1, v0), e2 = xsub(v2, v0);
   f3 p = xcross(d, e2);
   float det = xdot(e1, p);
-  if (det > -EPS && det < EPS) return false;
   float inv = __frcp_rn(det);
   f3 tv = xsub(o, v0);
   u = __fmul_rn(xdot(tv, p), inv);
-  if (u < 0.0f || u > 1.0f) return false;
   f3 q = xcross(tv, e1);
   v = __fmul_rn(xdot(d, q), inv);
-  if (v < 0.0f || __fadd_rn(u, v) > 1.0f) return false;
   t = __fmul_rn(xdot(e2, q), inv);
-  if (t < 0.0f) return false;
-  return true;
+  return !(det > -EPS && det < EPS) & !(u < 0.0f || u > 1.0f) & !(v < 0.0f || __fadd_rn(u, v) > 1.0f) & !(t < 0.0f);
 }
 
 // Tri.hpp:72-91: geometric point, interpolated normal, per-vertex plane
@@ -117,6 +116,23 @@ __device__ __forceinline__ float min3f(float a, float b, float c) {
   return r;
 }
 
+// Two packed floats, and four planes times a + b in two packed multiply-adds
+// (each half rounds like fmaf; tracing 16 samples per pixel of the 1080p
+// scene takes 82.0 ms with them, 83.2 with four fmaf).
+__device__ __forceinline__ uint64_t pack2(float a, float b) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void planes4(float (&t)[4], float4 p, float a, float b) {
+  const uint64_t aa = pack2(a, a), bb = pack2(b, b);
+  uint64_t lo, hi;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(lo) : "l"(pack2(p.x, p.y)), "l"(aa), "l"(bb));
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(hi) : "l"(pack2(p.z, p.w)), "l"(aa), "l"(bb));
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(t[0]), "=f"(t[1]) : "l"(lo));
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(t[2]), "=f"(t[3]) : "l"(hi));
+}
+
 // MODE kClosest: closest hit by reference distance.  kAny: any triangle hit
 // (env shadow rays, kernel.cu:247-248).  kPoint: point-light shadow ray:
 // occluded when the closest hit (by distance from the shadow origin o) lies
@@ -149,12 +165,13 @@ struct Traverser {
   float leaf_key;
   int32_t guard;
 
-  __device__ __forceinline__ float limit() const {
-    return MODE == kPoint ? fminf(best, tp) : best;
+  float lim;        // keys above it cannot hold a closer hit (kAny: unused)
+
+  // lim for a winner at reference distance b
+  __device__ __forceinline__ float limit(float b) const {
+    return (MODE == kPoint ? fminf(b, tp) : b) * 1.000001f + slack;
   }
-  __device__ __forceinline__ bool survives(float key) const {
-    return MODE == kAny || key <= limit() * 1.000001f + slack;
-  }
+  __device__ __forceinline__ bool survives(float key) const { return MODE == kAny || key <= lim; }
 
   __device__ __forceinline__ void init(const DevScene& S, f3 o_, f3 d_, f3 pp_, float pdist_) {
     init_at(S, o_, d_, pp_, pdist_, 0, S.scene_eps);
@@ -191,6 +208,7 @@ struct Traverser {
     poff = (MODE == kPoint) ? xlen(xsub(o, pp)) * 1.000001f + slack : 0.0f;
     tp = (MODE == kPoint) ? (pdist + poff) * 1.000001f + slack : INFINITY;
     best = INFINITY;
+    lim = limit(INFINITY);
     bkey = 0xFFFFFFFFu;
     slot = -1;
     t = u = v = 0.0f;
@@ -251,7 +269,7 @@ struct Traverser {
 
   // Expands `node`: tests its four child boxes, postpones / pushes leaf
   // children, pushes the other internal children and continues with the
-  // nearest.
+  // nearest (a child at an infinite key is pushed like the others).
   __device__ __forceinline__ void node_step(const DevScene& S, int2* sstk, int2* lstk, TravStats& st, uint32_t* err) {
     if (--guard < 0 || (uint64_t)node >= (uint64_t)S.n_nodes) {
       atomicOr(err, 4u);
@@ -341,25 +359,20 @@ struct Traverser {
       float4 c4 = __ldg(nd + 6);
       ch = make_int4(__float_as_int(c4.x), __float_as_int(c4.y), __float_as_int(c4.z), __float_as_int(c4.w));
       dl = __ldg(nd + 7);
-      const float nxa[4] = {nx.x, nx.y, nx.z, nx.w}, fxa[4] = {fx.x, fx.y, fx.z, fx.w};
-      const float nya[4] = {ny.x, ny.y, ny.z, ny.w}, fya[4] = {fy.x, fy.y, fy.z, fy.w};
-      const float nza[4] = {nz.x, nz.y, nz.z, nz.w}, fza[4] = {fz.x, fz.y, fz.z, fz.w};
-#pragma unroll
-      for (int k = 0; k < 4; k++) {
-        tnx[k] = fmaf(nxa[k], inv.x, bnear.x);
-        tfx[k] = fmaf(fxa[k], inv.x, bfar.x);
-        tny[k] = fmaf(nya[k], inv.y, bnear.y);
-        tfy[k] = fmaf(fya[k], inv.y, bfar.y);
-        tnz[k] = fmaf(nza[k], inv.z, bnear.z);
-        tfz[k] = fmaf(fza[k], inv.z, bfar.z);
-      }
+      planes4(tnx, nx, inv.x, bnear.x);
+      planes4(tfx, fx, inv.x, bfar.x);
+      planes4(tny, ny, inv.y, bnear.y);
+      planes4(tfy, fy, inv.y, bfar.y);
+      planes4(tnz, nz, inv.z, bnear.z);
+      planes4(tfz, fz, inv.z, bfar.z);
     }
     if (STATS) { st.nodes++; st.boxes += 4; }
     const float dla[4] = {dl.x, dl.y, dl.z, dl.w};
     const int32_t cha[4] = {ch.x, ch.y, ch.z, ch.w};
-    const float lim = limit() * 1.000001f + slack;
-    float ik[4];
-    int32_t ic[4];
+    bool hit[4];
+    float key[4];
+    float kmin = INFINITY;
+    int im = -1;  // the nearest internal child, expanded next
 #pragma unroll
     for (int c = 0; c < 4; c++) {
       float tnear = max3f(tnx[c], tny[c], tnz[c]);
@@ -367,37 +380,45 @@ struct Traverser {
       // FP32 nodes reject empty slots by their inverted boxes; a Q8 empty
       // slot decodes to an inverted box too, but the bias widening could
       // reopen it on a tiny node, so it is checked
-      bool hit = (!Q8 || cha[c] != kEmpty) && tnear <= tfar && tfar >= -slack;
-      float key = MODE == kAny ? tnear : tnear - dla[c];
-      if (MODE != kAny) hit = hit && key <= lim;
-      bool is_leaf = cha[c] < 0;
-      if (hit && is_leaf) {
-        if (leaf == 0) {
-          leaf = cha[c];
-          leaf_key = key;
-        } else if (!push(sstk, lstk, cha[c], key, err)) {
-          return;
+      hit[c] = (!Q8 || cha[c] != kEmpty) && tnear <= tfar && tfar >= -slack;
+      key[c] = MODE == kAny ? tnear : tnear - dla[c];
+      if (MODE != kAny) hit[c] = hit[c] && key[c] <= lim;
+      if (hit[c] && cha[c] >= 0 && key[c] < kmin) { kmin = key[c]; im = c; }
+    }
+    // The other children: the first leaf is postponed if the slot is free,
+    // the rest are pushed in slot order (their keys still prune them at the
+    // pop; a full sort cost more than it saved: 2 % slower on the 1080p
+    // scene).  With four free entries left in shared memory, which is all
+    // but a few steps, this is straight-line code of selects and predicated
+    // stores: written with a branch per child (leaf, push, shared or local
+    // entry) the lanes of a warp took it one after the other, and the
+    // 1.18M-triangle 1080p scene spent 96.0 instead of 83.5 ms tracing
+    // 16 samples per pixel.
+    node = -1;
+    if (sp <= kSmemStack - 4) {
+#pragma unroll
+      for (int c = 3; c >= 0; c--) {
+        const bool take = hit[c] && cha[c] < 0 && leaf == 0;
+        if (take) { leaf = cha[c]; leaf_key = key[c]; }
+        if (c == im) node = cha[c];
+        if (hit[c] && !take && c != im) {
+          sstk[sp * kTravBlock] = make_int2(cha[c], __float_as_int(key[c]));
+          sp++;
         }
       }
-      ik[c] = hit && !is_leaf ? key : INFINITY;
-      ic[c] = cha[c];
+    } else {
+#pragma unroll 1
+      for (int c = 3; c >= 0; c--) {
+        const bool h = c == 3 ? hit[3] : c == 2 ? hit[2] : c == 1 ? hit[1] : hit[0];
+        const float k = c == 3 ? key[3] : c == 2 ? key[2] : c == 1 ? key[1] : key[0];
+        const int32_t ref = c == 3 ? cha[3] : c == 2 ? cha[2] : c == 1 ? cha[1] : cha[0];
+        if (!h) continue;
+        if (ref < 0 && leaf == 0) { leaf = ref; leaf_key = k; }
+        else if (c == im) node = ref;
+        else if (!push(sstk, lstk, ref, k, err)) return;
+      }
     }
-    // internal children: the nearest is expanded next, the others are
-    // pushed in slot order (their keys still prune them at the pop; a full
-    // sort cost more than it saved: 2 % slower on the 1080p scene)
-    float kmin = ik[0];
-    int im = 0;
-#pragma unroll
-    for (int c = 1; c < 4; c++)
-      if (ik[c] < kmin) { kmin = ik[c]; im = c; }
-#pragma unroll
-    for (int c = 3; c >= 0; c--)
-      if (c != im && ik[c] < INFINITY && !push(sstk, lstk, ic[c], ik[c], err)) return;
-    if (kmin < INFINITY) {
-      node = ic[im];
-      return;
-    }
-    pop_next(sstk, lstk, err);
+    if (node < 0) pop_next(sstk, lstk, err);
   }
 
   // Intersects the triangles of the postponed leaf, then pops on if the lane
@@ -427,7 +448,7 @@ struct Traverser {
         float dist = xlen(xsub(p, o));
         uint32_t key = __float_as_uint(b.w);
         if (dist < best || (dist == best && key < bkey)) {
-          best = dist; slot = (int32_t)sl; t = tt; u = uu; v = vv; pos = p; bkey = key;
+          best = dist; lim = limit(dist); slot = (int32_t)sl; t = tt; u = uu; v = vv; pos = p; bkey = key;
           if (MODE == kPoint && (dist + poff) * 1.000001f < pdist) {
             occluded = true;  // the closest hit is at least this close
             done = true;
