@@ -213,7 +213,7 @@ __device__ __forceinline__ void flush_counts(unsigned long long* stats, int k, c
 // schedule runs them as three launches, the launch with phase 1 first.
 template <bool Q8, bool STATS, bool BATCH>
 __global__ void __launch_bounds__(kTravBlock, kTravMinBlocks)
-    k_trace(DevScene S, WaveView w, int32_t b, uint32_t* err, BatchView B, uint32_t phases) {
+    k_trace(DevScene S, WaveView w, int32_t b, uint32_t* err, BatchView B, uint32_t phases, int32_t min_width) {
   __shared__ int2 stk[kSmemStack * kTravBlock];
   const int32_t q = b & 1, qp = q ^ 1;
   const int32_t n_ext = (phases & 1u) ? w.counts[kExt + q] : 0;
@@ -237,8 +237,9 @@ __global__ void __launch_bounds__(kTravBlock, kTravMinBlocks)
   uint8_t* vis = w.vis;
   const int64_t half = w.shadow_half;
   TravStats st{0, 0, 0}, ss{0, 0, 0};
+  const int32_t width = rays_per_warp((int64_t)n_ext + n_pt + n_env, gridDim.x * (kTravBlock / 32), min_width);
   persistent_traverse<kClosest, Q8, STATS>(
-      S, n_ext, &w.counts[kClaim], stk + threadIdx.x, st, err,
+      S, n_ext, &w.counts[kClaim], stk + threadIdx.x, st, err, width,
       [&](int32_t i, auto& tr) {
         float4 a = qo[i], d = qd[i];
         if (BATCH) {
@@ -251,7 +252,7 @@ __global__ void __launch_bounds__(kTravBlock, kTravMinBlocks)
       [&](int32_t i, auto& tr) { hits[i] = make_float4(tr.t, tr.u, tr.v, __int_as_float(tr.slot)); });
   // point-light rays: shadow queue [half, half + n_pt)
   persistent_traverse<kPoint, Q8, STATS>(
-      S, n_pt, &w.counts[kClaim + 1], stk + threadIdx.x, ss, err,
+      S, n_pt, &w.counts[kClaim + 1], stk + threadIdx.x, ss, err, width,
       [&](int32_t i, auto& tr) {
         float4 a = so[half + i], d = sd[half + i], p = spp[half + i];
         if (BATCH) {
@@ -264,7 +265,7 @@ __global__ void __launch_bounds__(kTravBlock, kTravMinBlocks)
       [&](int32_t i, auto& tr) { vis[__float_as_int(so[half + i].w)] = tr.occluded ? 0 : 1; });
   // env rays: shadow queue [0, n_env)
   persistent_traverse<kAny, Q8, STATS>(
-      S, n_env, &w.counts[kClaim + 2], stk + threadIdx.x, ss, err,
+      S, n_env, &w.counts[kClaim + 2], stk + threadIdx.x, ss, err, width,
       [&](int32_t i, auto& tr) {
         float4 a = so[i], d = sd[i];
         if (BATCH) {
@@ -775,6 +776,7 @@ er_status run(er_scene* s, const er_render_opts* o, float* dump_rad, int32_t* du
   // accumulate(k) waits for accumulate(k - 1), so the film sees the samples
   // in index order as with one stream.
   const bool two = !dump_rad && !prof && !(o->flags & ER_RENDER_ONE_STREAM) && o->spp > sw;
+  const int32_t min_width = two ? 32 : kLoneWidth;
   if (two) {
     if ((st = ensure_wave2(s)) != ER_OK) return st;
     ER_CUDA(cudaEventRecord(s->ev_fork, s->stream));
@@ -827,10 +829,10 @@ er_status run(er_scene* s, const er_render_opts* o, float* dump_rad, int32_t* du
     for (int32_t b = 0; b <= max_depth; b++) {
       uint32_t* err = s->err_word;
       switch (variant) {
-        case 0: k_trace<false, false, false><<<g_tr[0], kTravBlock, 0, strm>>>(s->dev, w, b, err, NB, 7u); break;
-        case 1: k_trace<true, false, false><<<g_tr[1], kTravBlock, 0, strm>>>(s->dev, w, b, err, NB, 7u); break;
-        case 2: k_trace<false, true, false><<<g_tr[2], kTravBlock, 0, strm>>>(s->dev, w, b, err, NB, 7u); break;
-        default: k_trace<true, true, false><<<g_tr[3], kTravBlock, 0, strm>>>(s->dev, w, b, err, NB, 7u); break;
+        case 0: k_trace<false, false, false><<<g_tr[0], kTravBlock, 0, strm>>>(s->dev, w, b, err, NB, 7u, min_width); break;
+        case 1: k_trace<true, false, false><<<g_tr[1], kTravBlock, 0, strm>>>(s->dev, w, b, err, NB, 7u, min_width); break;
+        case 2: k_trace<false, true, false><<<g_tr[2], kTravBlock, 0, strm>>>(s->dev, w, b, err, NB, 7u, min_width); break;
+        default: k_trace<true, true, false><<<g_tr[3], kTravBlock, 0, strm>>>(s->dev, w, b, err, NB, 7u, min_width); break;
       }
       if ((st = mark(ER_STAGE_TRACE)) != ER_OK) return st;
       if (b == max_depth) break;
@@ -946,6 +948,7 @@ er_status render_backward_device(er_scene* s, const er_render_opts* o, const Gra
   // waves alternate between two pipelines as in run(); the gradients are
   // atomic sums, so the waves need no order between them
   const bool two = o->spp > sw;
+  const int32_t min_width = two ? 32 : kLoneWidth;
   if (two) {
     if ((st = ensure_wave2(s, true)) != ER_OK) return st;
     ER_CUDA(cudaEventRecord(s->ev_fork, s->stream));
@@ -971,9 +974,9 @@ er_status render_backward_device(er_scene* s, const er_render_opts* o, const Gra
     k_raygen<false, true><<<(n + 255) / 256, 256, 0, strm>>>(s->dev, w, P, n, NB, G);
     for (int32_t b = 0; b <= max_depth; b++) {
       if (s->dev.use_q8)
-        k_trace<true, false, false><<<g_tr[1], kTravBlock, 0, strm>>>(s->dev, w, b, s->err_word, NB, 7u);
+        k_trace<true, false, false><<<g_tr[1], kTravBlock, 0, strm>>>(s->dev, w, b, s->err_word, NB, 7u, min_width);
       else
-        k_trace<false, false, false><<<g_tr[0], kTravBlock, 0, strm>>>(s->dev, w, b, s->err_word, NB, 7u);
+        k_trace<false, false, false><<<g_tr[0], kTravBlock, 0, strm>>>(s->dev, w, b, s->err_word, NB, 7u, min_width);
       if (b == max_depth) break;
       k_shade<false, true><<<g_sh, 128, 0, strm>>>(s->dev, w, P, b, NB, G);
     }
@@ -1045,8 +1048,8 @@ er_status batch_launch(const DevScene& S, Wave* wv, const BatchSeg* d_segs, cons
     const WaveView& w = wk->v;
     cudaStream_t strm = alt ? pair->s2 : stream;
     auto trace = [&](int32_t b, const BatchView& B, uint32_t phases) {
-      if (q8) k_trace<true, false, true><<<g_tr, kTravBlock, 0, strm>>>(S, w, b, err, B, phases);
-      else k_trace<false, false, true><<<g_tr, kTravBlock, 0, strm>>>(S, w, b, err, B, phases);
+      if (q8) k_trace<true, false, true><<<g_tr, kTravBlock, 0, strm>>>(S, w, b, err, B, phases, two ? 32 : kLoneWidth);
+      else k_trace<false, false, true><<<g_tr, kTravBlock, 0, strm>>>(S, w, b, err, B, phases, two ? 32 : kLoneWidth);
       nl++;
     };
     if (bw.n_paths > wk->cap) return fail(ER_ERR_INVALID_ARG, "batch wave larger than its buffers");
@@ -1443,9 +1446,9 @@ extern "C" er_status er_render_noalloc(er_scene* s, const er_render_opts* o, flo
       k_raygen<false><<<(n + 255) / 256, 256, 0, s->stream>>>(s->dev, w, P, n, NB, GradArgs{});  // also zeroes the queue counters
       for (int32_t b = 0; b <= max_depth; b++) {
         if (s->dev.use_q8)
-          k_trace<true, false, false><<<g_tr8, kTravBlock, 0, s->stream>>>(s->dev, w, b, s->err_word, NB, 7u);
+          k_trace<true, false, false><<<g_tr8, kTravBlock, 0, s->stream>>>(s->dev, w, b, s->err_word, NB, 7u, kLoneWidth);
         else
-          k_trace<false, false, false><<<g_tr, kTravBlock, 0, s->stream>>>(s->dev, w, b, s->err_word, NB, 7u);
+          k_trace<false, false, false><<<g_tr, kTravBlock, 0, s->stream>>>(s->dev, w, b, s->err_word, NB, 7u, kLoneWidth);
         if (b == max_depth) break;
         k_shade<false><<<g_sh, 128, 0, s->stream>>>(s->dev, w, P, b, NB, GradArgs{});
       }

@@ -14,6 +14,7 @@ __global__ void __launch_bounds__(kTravBlock, kTravMinBlocks)
   TravStats st{0, 0, 0};
   persistent_traverse<kClosest, Q8, STATS>(
       S, n, counter, stk + threadIdx.x, st, err,
+      rays_per_warp(n, gridDim.x * (kTravBlock / 32), kLoneWidth),
       [&](int32_t i, auto& tr) {
         const float* q = rays + 6 * (int64_t)i;
         f3 o = mk(q[0], q[1], q[2]);
@@ -39,7 +40,7 @@ __global__ void __launch_bounds__(kTravBlock, kTravMinBlocks)
 template <bool Q8, bool STATS>
 void launch(er_scene* s, const float* rays, int64_t n, int normalize, int32_t* tri, float* dist, float* uv) {
   const int grid = blocks_per_sm((const void*)k_trace_rays<Q8, STATS>, kTravBlock) * s->num_sms;
-  int64_t need = (n + kTravBlock - 1) / kTravBlock;
+  int64_t need = (n + kTravBlock / 32 * kLoneWidth - 1) / (kTravBlock / 32 * kLoneWidth);
   int g = (int)(need < grid ? need : grid);
   if (g < 1) g = 1;
   int32_t* counter = (int32_t*)((char*)s->err_word + 32);

@@ -473,20 +473,38 @@ constexpr int kRefillThreshold = ER_REFILL_THRESHOLD;
 // have no node left to expand (they would idle through node rounds).
 constexpr int kLeafRoundStuck = ER_LEAF_ROUND_STUCK;
 
+constexpr int32_t kLoneWidth = 4;  // fewest rays of a warp while no other wave runs
+// Rays a warp traces at a time, for a launch of n rays on n_warps resident
+// warps: 32, and fewer when that leaves more of the warps with work.  A
+// launch lasts as long as its slowest warp, and a warp of 32 different rays
+// takes its node and leaf rounds one after the other, so a small queue is
+// spread over the whole machine: 320x240 pixels of the 16-sphere scene at
+// one sample (76,800 rays on 4,256 warps) trace in 254 us with at least 4
+// rays per warp, 269 with 8, 316 with 32.  The same instructions fill fewer
+// lanes, so this pays only while nothing else runs: with a second wave in
+// flight (floor = 32) 641x479 at 9 samples takes 1.57 ms, with a floor of 4
+// 1.66 ms.  From 2 x 32 rays per resident warp on, all lanes are used.
+__device__ __forceinline__ int32_t rays_per_warp(int64_t n, int32_t n_warps, int32_t floor) {
+  return max(floor, (int32_t)min((int64_t)32, n / (2 * n_warps)));
+}
+
 // Persistent, warp-refilling traversal over a queue of n items.  `load(i,
 // tr)` initialises lane state for item i, `store(i, tr)` consumes a finished
 // traversal.  Items are claimed in warp batches from *counter, which must be
-// zero at launch.
+// zero at launch.  Only the first `width` lanes of a warp take items
+// (rays_per_warp).
 template <int MODE, bool Q8, bool STATS, typename Load, typename Store>
 __device__ __forceinline__ void persistent_traverse(const DevScene& S, int32_t n, int32_t* counter, int2* sstk,
-                                                    TravStats& st, uint32_t* err, Load load, Store store) {
+                                                    TravStats& st, uint32_t* err, int32_t width, Load load,
+                                                    Store store) {
   // An empty queue claims nothing, so its counter stays zero for a later
   // launch of the same phase.
   if (n <= 0) return;
   int2 lstk[kLocalStack];
   Traverser<MODE, Q8, STATS> tr;
   const unsigned lane = threadIdx.x & 31u;
-  int32_t item = -1;  // -1: needs an item; >= n: queue exhausted
+  int32_t item = (int32_t)lane < width ? -1 : n;  // -1: needs an item; >= n: queue exhausted
+  const int32_t refill = min(kRefillThreshold, (width * 5) >> 3);
   bool active = false;
   while (true) {
     bool need = item < 0;
@@ -528,7 +546,7 @@ __device__ __forceinline__ void persistent_traverse(const DevScene& S, int32_t n
       }
       unsigned am = __ballot_sync(0xFFFFFFFFu, active);
       unsigned want = __ballot_sync(0xFFFFFFFFu, item < 0);
-      if (__popc(am) < kRefillThreshold && want) break;
+      if (__popc(am) < refill && want) break;
       if (!am) break;
     }
   }
