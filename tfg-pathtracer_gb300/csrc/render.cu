@@ -3,8 +3,8 @@
 //
 //   raygen -> [ extend (closest hit) -> shade -> shadow ] x max_depth -> accumulate
 //
-// One wave traces spp_wave samples of every pixel.  Paths are indexed
-// p = s * npix + pix; per-path state lives in SoA arrays, queues hold
+// One wave traces spp_wave samples of every pixel.  Paths are numbered in
+// groups of pixels (path_pixel); per-path state lives in SoA arrays, queues hold
 // (origin|path, direction) pairs and are appended with warp ballots + one
 // atomic per warp.  Radiance contributions of a vertex are resolved in the
 // reference's order (kernel.cu:351-357) once its two shadow rays are done,
@@ -135,22 +135,49 @@ __device__ __forceinline__ f3 sample_adjoint(f3 L, float4 g4, uint32_t n) {
             (keep && L.z > 0.f && L.z < 10.f) ? g4.z * inv_n : 0.f);
 }
 
-// Path order within a sample: 8x4 pixel tiles (a warp's 32 paths start in
-// one tile, so its primary rays and first hits are coherent) when the image
-// divides into them, else raster order.  pix = y * W + x either way; the
-// random numbers and the output slot depend only on the pixel, so the order
-// changes no result.
-__device__ __forceinline__ bool tiled(const WaveParams& P) { return (P.W & 7) == 0 && (P.H & 3) == 0; }
-__device__ __forceinline__ int32_t path_pixel(const WaveParams& P, int32_t q) {
-  if (!tiled(P)) return q;
-  const int32_t t = q >> 5, r = q & 31, tw = P.W >> 3;
-  const int32_t x = ((t % tw) << 3) + (r & 7), y = ((t / tw) << 2) + (r >> 3);
-  return y * P.W + x;
+// Pixels in tile order: 8x4 pixel tiles row by row (a warp's 32 pixels lie
+// in one tile, so its primary rays and first hits are coherent), then the
+// columns and rows left over when the image does not divide into tiles.
+// pix = y * W + x.
+__device__ __forceinline__ int32_t tile_pixel(const WaveParams& P, int32_t q) {
+  const int32_t tw = P.W >> 3, th = P.H >> 2, rest = P.W & 7;
+  if (q < tw * th * 32) {
+    const int32_t t = q >> 5, r = q & 31;
+    return (((t / tw) << 2) + (r >> 3)) * P.W + ((t % tw) << 3) + (r & 7);
+  }
+  q -= tw * th * 32;
+  if (q < rest * th * 4) return (q / rest) * P.W + (tw << 3) + q % rest;
+  return th * 4 * P.W + q - rest * th * 4;
 }
-__device__ __forceinline__ int32_t pixel_path(const WaveParams& P, int32_t pix) {
-  if (!tiled(P)) return pix;
-  const int32_t x = pix % P.W, y = pix / P.W;
-  return (((y >> 2) * (P.W >> 3) + (x >> 3)) << 5) + ((y & 3) << 3) + (x & 7);
+__device__ __forceinline__ int32_t pixel_tile(const WaveParams& P, int32_t pix) {
+  const int32_t x = pix % P.W, y = pix / P.W, tw = P.W >> 3, th = P.H >> 2, rest = P.W & 7;
+  if (y >= th * 4) return pix;
+  if (x >= tw << 3) return tw * th * 32 + y * rest + x - (tw << 3);
+  return (((y >> 2) * tw + (x >> 3)) << 5) + ((y & 3) << 3) + (x & 7);
+}
+
+// Path order of a slice: groups of four pixels in tile order, all samples
+// of a group together (the last group may have fewer pixels).  A warp of a
+// many-sample wave thus starts in one or two pixels, so its rays, hits,
+// materials and texels stay closer together for the whole path than those
+// of 32 pixels at one sample, and the rays in flight cover a smaller part
+// of the image.  Random numbers and output slots follow the pixel and
+// sample, so the order changes no result.  Against whole images sample
+// after sample (8x4 tiles only where the image divides into them): 512x512
+// at 64 samples, forward and gradient, 46.1 -> 42.1 ms, of which 43.8 with
+// groups of 32 pixels; 641x479 at 9 samples 1.71 -> 1.63 ms; 1080p at 16
+// samples 110.6 -> 108.7 ms.
+constexpr int kGroup = 2;  // log2 of the pixels per group
+__device__ __forceinline__ void path_pixel(const WaveParams& P, int32_t local, int32_t& pix, int32_t& s) {
+  const int32_t per = P.spp_wave << kGroup, g = local / per, r = local - g * per;
+  const int32_t c = min(1 << kGroup, P.npix - (g << kGroup));
+  s = r / c;
+  pix = tile_pixel(P, (g << kGroup) + r - s * c);
+}
+// Index within its slice of sample s of the q-th pixel in tile order.
+__device__ __forceinline__ int32_t path_index(const WaveParams& P, int32_t q, int32_t s) {
+  const int32_t g = q >> kGroup, c = min(1 << kGroup, P.npix - (g << kGroup));
+  return g * (P.spp_wave << kGroup) + s * c + (q & ((1 << kGroup) - 1));
 }
 
 template <bool BATCH, bool GRAD = false>
@@ -163,7 +190,8 @@ __global__ void k_raygen(DevScene S, WaveView w, WaveParams P, int32_t n, BatchV
   if (p >= n) return;
   int32_t job;
   int32_t local = path_slice<BATCH>(B, p, P, job);
-  int32_t pix = path_pixel(P, local % P.npix), s = local / P.npix;
+  int32_t pix, s;
+  path_pixel(P, local, pix, s);
   int32_t x = pix % P.W, y = pix / P.W;
   uint32_t idx = (uint32_t)out_index(P, x, y);
   uint32_t sample = (uint32_t)(P.sample_base + s);
@@ -399,7 +427,8 @@ __global__ void __launch_bounds__(128, GRAD ? kShadeGradMinBlocks : kShadeMinBlo
         L.z = __fadd_rn(L.z, __fmul_rn(e.z, thr.z));
         w.bounces[p] = bounce;
       } else {
-        int32_t pix = path_pixel(P, local % P.npix), s = local / P.npix;
+        int32_t pix, s;
+        path_pixel(P, local, pix, s);
         uint32_t idx = (uint32_t)out_index(P, pix % P.W, pix / P.W);
         VertexShade V;
         shade_vertex<BATCH || GRAD>(S, P.flags, P.k0, P.k1, idx, (uint32_t)(P.sample_base + s), bounce, o, d, h.x, h.y, h.z,
@@ -516,8 +545,9 @@ __device__ __forceinline__ void accumulate_pixel(const WaveView& w, const WavePa
   if (fp64) { s0 = F.sum[3 * (size_t)idx]; s1 = F.sum[3 * (size_t)idx + 1]; s2 = F.sum[3 * (size_t)idx + 2]; }
   float4 a[3];
   if (F.aov_on) for (int k = 0; k < 3; k++) a[k] = F.aov[k][idx];
+  const int32_t q = pixel_tile(P, pix);
   for (int32_t s = 0; s < sw; s++) {
-    int32_t p = path_base + s * P.npix + pixel_path(P, pix);
+    int32_t p = path_base + path_index(P, q, s);
     float4 L = w.light[p];
     resolve(w, p, L);
     if (F.keep) {
@@ -571,7 +601,8 @@ __global__ void k_dump(WaveView w, WaveParams P, int32_t sw, int32_t s_off, floa
   if (p >= sw * P.npix) return;
   float4 L = w.light[p];
   resolve(w, p, L);
-  int32_t pix = path_pixel(P, p % P.npix), s = p / P.npix;
+  int32_t pix, s;
+  path_pixel(P, p, pix, s);
   int64_t j = (int64_t)(s + s_off) * P.npix + out_index(P, pix % P.W, pix / P.W);
   rad[3 * j] = L.x; rad[3 * j + 1] = L.y; rad[3 * j + 2] = L.z;
   bnc[j] = w.bounces[p];
