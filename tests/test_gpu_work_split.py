@@ -53,3 +53,14 @@ def test_path_order(w, h, spp):
             for key in ("beauty", "normal", "samples", "pathcount"):
                 assert np.array_equal(cut[key], whole[key], equal_nan=True), (k, key)
         assert (whole["samples"] <= spp).all()
+
+
+def test_shade_groups():
+    """Waves of 0.3, 1.5 and 4.9 million paths (shade groups of 128 to 512 items) give the same film."""
+    arrays = scenes.config0(x_res=640, y_res=480)
+    with _lib.Scene(arrays) as s:
+        whole = s.render(16, max_depth=4, seed=2, spp_per_wave=16)
+        for k in (1, 5):
+            cut = s.render(16, max_depth=4, seed=2, spp_per_wave=k)
+            for key in ("beauty", "samples", "pathcount"):
+                assert np.array_equal(cut[key], whole[key], equal_nan=True), (k, key)

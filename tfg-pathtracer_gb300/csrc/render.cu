@@ -348,23 +348,57 @@ __device__ __forceinline__ void grad_prev_vertex(const WaveView& w, const GradAr
 #ifndef ER_SHADE_MIN_BLOCKS
 #define ER_SHADE_MIN_BLOCKS 7
 #endif
-#ifndef ER_SHADE_GRAD_MIN_BLOCKS
-#define ER_SHADE_GRAD_MIN_BLOCKS 12
-#endif
 // Resident 128-thread shade blocks per SM the register budgets are sized
-// for.  Both kernels wait on dependent loads (texture, material, env
-// lookups, atomics), so occupancy pays for some spilling.  Forward: 73
-// registers at 7 blocks (unbounded 117 at 4 blocks: 10 % longer stage on
-// the 1080p scene; 8 blocks spill too much).  Gradient: 42 registers at 12
-// blocks (unbounded 209 at 2 blocks): backward of the 512x512 adjoint
-// workload 34.9 vs 49.7 ms.
+// for (72 registers).  The kernels wait on dependent loads (texture, material,
+// env lookups, atomics), so occupancy pays for some spilling.  Forward:
+// unbounded 117 registers at 4 blocks, 10 % longer stage on the 1080p scene;
+// 6 and 8 blocks 27.2 ms against 24.6 for 16 samples.  Gradient: 512x512 at
+// 64 samples, forward and gradient, 37.7 ms at 7 blocks, 37.8 at 6, 38.4 at
+// 10, 38.8 at 12.
 constexpr int kShadeMinBlocks = ER_SHADE_MIN_BLOCKS;
-constexpr int kShadeGradMinBlocks = ER_SHADE_GRAD_MIN_BLOCKS;
+constexpr int kShadeBlock = 128;
+
+// The block's items base .. base + rounds * 128 (index n and beyond: none),
+// those whose ray hit something before those whose ray escaped: into s_item,
+// for the block to take 128 at a time.  Hits and escapes of a bounce after the
+// first lie mixed in the queue, and a warp that holds both runs the whole
+// vertex for its few hits and then the environment lookup for the others;
+// this leaves one mixed warp per block and group.  A block takes 4 x 128
+// items together when it has at least 8 such groups to do, so that the last
+// group costs little.  512x512 at 64 samples, forward and gradient: 36.1 ms,
+// with groups of 128 items 37.7, without 40.9 ms; groups of each warp alone
+// (no barrier, but the warps of a block drift apart in the code): 38.5.
+constexpr int kShadeRounds = 4;
+__device__ __forceinline__ void hits_first(const float4* hits, int32_t base, int32_t n, int32_t rounds,
+                                           int32_t* s_hits, int32_t* s_item) {
+  constexpr int32_t kWarps = kShadeBlock / 32;
+  const int32_t wp = threadIdx.x >> 5;
+  unsigned hm[kShadeRounds];
+#pragma unroll
+  for (int32_t r = 0; r < kShadeRounds; r++) {
+    const int32_t i = base + r * kShadeBlock + threadIdx.x;
+    hm[r] = __ballot_sync(0xFFFFFFFFu, r < rounds && i < n && __float_as_int(hits[i].w) >= 0);
+    if (lane_id() == 0) s_hits[r * kWarps + wp] = __popc(hm[r]);
+  }
+  // (also: every warp has taken its items of the previous group)
+  __syncthreads();
+  int32_t all = 0;
+  for (int32_t k = 0; k < kWarps * rounds; k++) all += s_hits[k];
+#pragma unroll
+  for (int32_t r = 0; r < kShadeRounds; r++) {
+    if (r >= rounds) break;
+    int32_t h = __popc(hm[r] & ((1u << lane_id()) - 1u));
+    for (int32_t k = 0; k < r * kWarps + wp; k++) h += s_hits[k];
+    const int32_t at = r * kShadeBlock + threadIdx.x;
+    s_item[(hm[r] >> lane_id()) & 1u ? h : all + at - h] = base + at;
+  }
+  __syncthreads();
+}
 
 // EVAL: the detached estimator of er_render_replay, BRDF values and
 // environment radiance from G's evaluation parameters.
 template <bool BATCH, bool GRAD = false, bool EVAL = false>
-__global__ void __launch_bounds__(128, GRAD ? kShadeGradMinBlocks : kShadeMinBlocks)
+__global__ void __launch_bounds__(kShadeBlock, kShadeMinBlocks)
     k_shade(DevScene S0, WaveView w, WaveParams P0, int32_t bounce, BatchView B, GradArgs G) {
   const int32_t qin = bounce & 1;
   const int32_t n = w.counts[kExt + qin];
@@ -376,8 +410,17 @@ __global__ void __launch_bounds__(128, GRAD ? kShadeGradMinBlocks : kShadeMinBlo
     w.counts[kClaim + 1] = 0;
     w.counts[kClaim + 2] = 0;
   }
-  for (int32_t base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x) {
-    int32_t i = base + threadIdx.x;
+  __shared__ int32_t s_item[kShadeRounds * kShadeBlock];
+  __shared__ int32_t s_hits[kShadeRounds * kShadeBlock / 32];
+  const int32_t rounds = min(kShadeRounds, max(1, n / (8 * kShadeBlock * (int32_t)gridDim.x)));
+  const int32_t per = rounds * kShadeBlock;
+  for (int32_t base = blockIdx.x * per, round = 0; base < n;) {
+    if (round == 0) hits_first(w.hits, base, n, rounds, s_hits, s_item);
+    const int32_t i = s_item[round * kShadeBlock + threadIdx.x];
+    if (++round == rounds) {
+      round = 0;
+      base += gridDim.x * per;
+    }
     bool valid = i < n;
     bool push_next = false, push_env = false, push_pt = false;
     f3 next_o = mk1(0), next_d = mk1(0), env_o = mk1(0), env_d = mk1(0), pt_o = mk1(0), pt_d = mk1(0),
