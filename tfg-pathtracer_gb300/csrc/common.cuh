@@ -45,6 +45,48 @@ __device__ __forceinline__ f3 xnormalize(f3 a) {
   return mk(__fdiv_rn(a.x, l), __fdiv_rn(a.y, l), __fdiv_rn(a.z, l));
 }
 
+// -------------------------------------------------------- pairs of floats --
+//
+// h + l with |l| <= ulp(h) / 2 (T. J. Dekker, "A floating-point technique
+// for extending the available precision", Numer. Math. 18, 1971): expressions
+// the reference evaluates in double, at a sixty-fourth of the FP32 rate here,
+// are computed in pairs and rounded to float by settled(), which says whether
+// the rounding could have come out otherwise (A. Ziv, "Fast evaluation of
+// elementary mathematical functions with correctly rounded last bit", ACM
+// TOMS 17, 1991).  About one value in 2^16 cannot be told, and is evaluated in
+// double; so the results are the same bits.
+struct ff {
+  float h, l;
+};
+__device__ __forceinline__ ff two_sum(float a, float b) {  // |a| >= |b|
+  const float s = __fadd_rn(a, b);
+  return {s, __fsub_rn(b, __fsub_rn(s, a))};
+}
+__device__ __forceinline__ ff two_prod(float a, float b) {
+  const float p = __fmul_rn(a, b);
+  return {p, __fmaf_rn(a, b, -p)};
+}
+__device__ __forceinline__ ff mul(ff a, ff b) {
+  const ff p = two_prod(a.h, b.h);
+  return two_sum(p.h, __fmaf_rn(a.h, b.l, __fmaf_rn(a.l, b.h, p.l)));
+}
+__device__ __forceinline__ ff mul(ff a, float b) {
+  const ff p = two_prod(a.h, b);
+  return two_sum(p.h, __fmaf_rn(a.l, b, p.l));
+}
+// a + b for a.h >= b >= 0 or b >= a.h >= 0
+__device__ __forceinline__ ff add(ff a, float b) {
+  const ff s = a.h >= b ? two_sum(a.h, b) : two_sum(b, a.h);
+  return two_sum(s.h, __fadd_rn(s.l, a.l));
+}
+// The float nearest to h + l (l small against h) if it is the same for
+// every value within 2^-41 of it.
+__device__ __forceinline__ bool settled(float h, float l, float* r) {
+  const float e = __fmul_rn(fabsf(h), 0x1p-41f);
+  *r = __fadd_rn(h, __fadd_rn(l, e));
+  return *r == __fadd_rn(h, __fsub_rn(l, e));
+}
+
 // ------------------------------------------------------------ fast ops --
 __device__ __forceinline__ f3 operator+(f3 a, f3 b) { return mk(a.x + b.x, a.y + b.y, a.z + b.z); }
 __device__ __forceinline__ f3 operator-(f3 a, f3 b) { return mk(a.x - b.x, a.y - b.y, a.z - b.z); }

@@ -147,6 +147,7 @@ struct DevCamera {
   float focal_length, sensor_width, sensor_height, aperture, focus_distance;
   float px, py, pz;
   float cx, sx, cy, sy, cz, sz;  // cosf / sinf of the rotation in radians
+  float px_h, px_l, py_h, py_l;  // 1.0 / x_res and 1.0 / y_res as pairs of floats
   int32_t bokeh;
 };
 

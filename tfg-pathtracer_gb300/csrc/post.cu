@@ -14,6 +14,7 @@
 #include <cstring>
 #include <vector>
 
+#include "common.cuh"
 #include "internal.h"
 
 namespace er {
@@ -45,38 +46,6 @@ __device__ __forceinline__ float clampr(float a, float b, float c) { return a < 
 //    compared with the double expressions for every float of [2^-20, 2^17)
 //    and [2^-12, 2^5): no difference;
 //  - the encoding in integers.
-
-struct ff {  // h + l, |l| <= ulp(h) / 2
-  float h, l;
-};
-__device__ __forceinline__ ff two_sum(float a, float b) {  // |a| >= |b|
-  const float s = __fadd_rn(a, b);
-  return {s, __fsub_rn(b, __fsub_rn(s, a))};
-}
-__device__ __forceinline__ ff two_prod(float a, float b) {
-  const float p = __fmul_rn(a, b);
-  return {p, __fmaf_rn(a, b, -p)};
-}
-__device__ __forceinline__ ff mul(ff a, ff b) {
-  const ff p = two_prod(a.h, b.h);
-  return two_sum(p.h, __fmaf_rn(a.h, b.l, __fmaf_rn(a.l, b.h, p.l)));
-}
-__device__ __forceinline__ ff mul(ff a, float b) {
-  const ff p = two_prod(a.h, b);
-  return two_sum(p.h, __fmaf_rn(a.l, b, p.l));
-}
-// a + b for a.h >= b >= 0 or b >= a.h >= 0
-__device__ __forceinline__ ff add(ff a, float b) {
-  const ff s = a.h >= b ? two_sum(a.h, b) : two_sum(b, a.h);
-  return two_sum(s.h, __fadd_rn(s.l, a.l));
-}
-// The float nearest to h + l (l small against h) if it is the same for
-// every value within 2^-41 of it.
-__device__ __forceinline__ bool settled(float h, float l, float* r) {
-  const float e = __fmul_rn(fabsf(h), 0x1p-41f);
-  *r = __fadd_rn(h, __fadd_rn(l, e));
-  return *r == __fadd_rn(h, __fsub_rn(l, e));
-}
 
 __device__ __noinline__ float aces_exact(float x) {
   const float a = 2.51f, b = 0.03f, c = 2.43f, d = 0.59f, e = 0.14f;

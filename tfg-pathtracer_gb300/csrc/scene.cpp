@@ -54,6 +54,11 @@ DevCamera make_dev_camera(const er_camera& c) {
   d.cx = cosf(rx); d.sx = sinf(rx);
   d.cy = cosf(ry); d.sy = sinf(ry);
   d.cz = cosf(rz); d.sz = sinf(rz);
+  const double ix = 1.0 / (double)(float)c.x_res, iy = 1.0 / (double)(float)c.y_res;
+  d.px_h = (float)ix;
+  d.px_l = (float)(ix - (double)d.px_h);
+  d.py_h = (float)iy;
+  d.py_l = (float)(iy - (double)d.py_h);
   d.bokeh = c.bokeh;
   return d;
 }
