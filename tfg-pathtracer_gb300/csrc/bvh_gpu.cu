@@ -242,120 +242,218 @@ __device__ __forceinline__ void refit(BNode* nodes, const float* pos, const int3
   b.cost = kSahNode * area_of(b.lo, b.hi) + l.cost + r.cost;
 }
 
+// A treelet as the lanes of its warp share it.
+struct Treelet {
+  float lo[kTreelet][3], hi[kTreelet][3], delta[kTreelet];
+  int32_t count[kTreelet], leaf[kTreelet];
+  int32_t inner[kTreelet - 1];           // its internal nodes, the root first
+  float cost[1 << kTreelet];             // least cost of each leaf subset
+  uint8_t part[1 << kTreelet];           // the side of the best split that holds the lowest leaf
+  int32_t node[kTreelet - 1], left[kTreelet - 1], right[kTreelet - 1];  // the rebuilt nodes
+  uint8_t mask[kTreelet - 1];
+};
+
+// The subsets of seven leaves with two to five elements, by size.
+__device__ const uint8_t kSubsets[112] = {
+    3,   5,   6,   9,   10,  12,  17,  18,  20,  24,  33,  34,  36,  40,  48,  65,  66,  68,  72,  80,  96,
+    7,   11,  13,  14,  19,  21,  22,  25,  26,  28,  35,  37,  38,  41,  42,  44,  49,  50,  52,  56,  67,  69,  70,
+    73,  74,  76,  81,  82,  84,  88,  97,  98,  100, 104, 112,
+    15,  23,  27,  29,  30,  39,  43,  45,  46,  51,  53,  54,  57,  58,  60,  71,  75,  77,  78,  83,  85,  86,  89,
+    90,  92,  99,  101, 102, 105, 106, 108, 113, 114, 116, 120,
+    31,  47,  55,  59,  61,  62,  79,  87,  91,  93,  94,  103, 107, 109, 110, 115, 117, 118, 121, 122, 124};
+
+// Restructures the treelet rooted at node `cur`, all lanes of a warp together.
+__device__ void restructure(const float* pos, const int32_t* sorted, const float* tdelta, BNode* nodes,
+                            int32_t* leaf_parent, int32_t cur, Treelet& W) {
+  const int lane = threadIdx.x & 31;
+  const unsigned all = 0xFFFFFFFFu;
+  // lane j holds leaf j of the treelet; it grows by opening the largest
+  // internal leaf (the first of equals)
+  int32_t ref = lane == 0 ? __ldcg(&nodes[cur].left) : lane == 1 ? __ldcg(&nodes[cur].right) : 0;
+  Sub sub;
+  for (int a = 0; a < 3; a++) sub.lo[a] = sub.hi[a] = 0.f;
+  sub.delta = sub.cost = 0.f;
+  sub.count = 0;
+  if (lane < 2) sub = sub_of(nodes, pos, sorted, tdelta, ref);
+  float rlo[3], rhi[3];
+  for (int a = 0; a < 3; a++) {
+    rlo[a] = fminf(__shfl_sync(all, sub.lo[a], 0), __shfl_sync(all, sub.lo[a], 1));
+    rhi[a] = fmaxf(__shfl_sync(all, sub.hi[a], 0), __shfl_sync(all, sub.hi[a], 1));
+  }
+  const float now =
+      kSahNode * area_of(rlo, rhi) + __shfl_sync(all, sub.cost, 0) + __shfl_sync(all, sub.cost, 1);
+  if (lane == 0) W.inner[0] = cur;
+  int nt = 2;
+  while (nt < kTreelet) {
+    const unsigned key = lane < nt && ref >= 0 ? __float_as_uint(area_of(sub.lo, sub.hi)) + 1u : 0u;
+    const unsigned top = __reduce_max_sync(all, key);
+    if (top == 0) break;
+    const int pick = __ffs(__ballot_sync(all, key == top)) - 1;
+    const int32_t t = __shfl_sync(all, ref, pick);
+    if (lane == 0) W.inner[nt - 1] = t;
+    if (lane == pick) ref = __ldcg(&nodes[t].left);
+    if (lane == nt) ref = __ldcg(&nodes[t].right);
+    if (lane == pick || lane == nt) sub = sub_of(nodes, pos, sorted, tdelta, ref);
+    nt++;
+  }
+  if (lane < nt) {
+    for (int a = 0; a < 3; a++) { W.lo[lane][a] = sub.lo[a]; W.hi[lane][a] = sub.hi[a]; }
+    W.delta[lane] = sub.delta;
+    W.count[lane] = sub.count;
+    W.leaf[lane] = ref;
+    W.cost[1 << lane] = sub.cost;
+  }
+  __syncwarp();
+  // bounds of leaf subset s
+  auto bounds = [&](int s, float* lo, float* hi) {
+    for (int a = 0; a < 3; a++) { lo[a] = INFINITY; hi[a] = -INFINITY; }
+    for (int j = 0; j < kTreelet; j++)
+      if (s >> j & 1)
+        for (int a = 0; a < 3; a++) { lo[a] = fminf(lo[a], W.lo[j][a]); hi[a] = fmaxf(hi[a], W.hi[j][a]); }
+  };
+  auto node_cost = [&](int s) {
+    float lo[3], hi[3];
+    bounds(s, lo, hi);
+    return kSahNode * area_of(lo, hi);
+  };
+  // least-cost topology: subsets of two to five leaves, a lane each, then the
+  // larger ones with their splits over the lanes; the split is {lowest leaf | q,
+  // the rest}, the largest q of equals
+  const int full = (1 << nt) - 1;
+  constexpr int first[5] = {0, 21, 56, 91, 112};
+  for (int size = 2; size <= 5 && size <= nt; size++) {
+    for (int e = first[size - 2] + lane; e < first[size - 1]; e += 32) {
+      const int s = kSubsets[e];
+      if (s > full) break;  // (ascending within a size)
+      const int low = s & -s, rest = s ^ low;
+      float best = INFINITY;
+      int bp = low;
+      for (int q = (rest - 1) & rest;; q = (q - 1) & rest) {
+        const int pp = low | q;
+        const float c = W.cost[pp] + W.cost[s ^ pp];
+        if (c < best) { best = c; bp = pp; }
+        if (q == 0) break;
+      }
+      W.cost[s] = node_cost(s) + best;
+      W.part[s] = (uint8_t)bp;
+    }
+    __syncwarp();
+  }
+  for (int size = 6; size <= nt; size++) {
+    for (int j = 0; j < (size == nt ? 1 : nt); j++) {
+      const int s = size == nt ? full : full ^ (1 << j);
+      const int low = s & -s, rest = s ^ low;
+      float best = INFINITY;
+      int bq = 0;
+      for (int k = lane; k < (1 << (size - 1)) - 1; k += 32) {
+        int q = 0, bit = 0;
+        for (int m = rest; m; m &= m - 1, bit++)
+          if (k >> bit & 1) q |= m & -m;
+        const float c = W.cost[low | q] + W.cost[s ^ (low | q)];
+        if (c < best || (c == best && q > bq)) { best = c; bq = q; }
+      }
+      const unsigned bits = __float_as_uint(best), least = __reduce_min_sync(all, bits);
+      const int q = (int)__reduce_max_sync(all, bits == least ? (unsigned)bq : 0u);
+      if (lane == 0) {
+        W.cost[s] = node_cost(s) + __uint_as_float(least);
+        W.part[s] = (uint8_t)(low | q);
+      }
+    }
+    __syncwarp();
+  }
+  if (!(W.cost[full] < now * (1.0f - 1e-6f))) {
+    if (lane == 0) nodes[cur].cost = now;
+    return;
+  }
+  // rebuild with the treelet's internal nodes, parents first
+  if (lane == 0) {
+    int st_s[kTreelet], st_o[kTreelet];
+    int sp = 0, used = 1, no = 1;
+    W.node[0] = cur;
+    st_s[sp] = full;
+    st_o[sp++] = 0;
+    while (sp > 0) {
+      const int sset = st_s[--sp], o = st_o[sp];
+      W.mask[o] = (uint8_t)sset;
+      const int sides[2] = {W.part[sset], sset ^ W.part[sset]};
+      int32_t ch[2];
+      for (int c = 0; c < 2; c++) {
+        if ((sides[c] & (sides[c] - 1)) == 0) {
+          ch[c] = W.leaf[__ffs(sides[c]) - 1];
+        } else {
+          ch[c] = W.inner[used++];
+          W.node[no] = ch[c];
+          st_s[sp] = sides[c];
+          st_o[sp++] = no++;
+        }
+      }
+      W.left[o] = ch[0];
+      W.right[o] = ch[1];
+    }
+  }
+  __syncwarp();
+  if (lane < nt - 1) {
+    const int32_t nd = W.node[lane];
+    const int s = W.mask[lane];
+    BNode& b = nodes[nd];
+    float lo[3], hi[3], dl = 0.f;
+    int32_t cnt = 0;
+    bounds(s, lo, hi);
+    for (int j = 0; j < kTreelet; j++)
+      if (s >> j & 1) { dl = fmaxf(dl, W.delta[j]); cnt += W.count[j]; }
+    for (int a = 0; a < 3; a++) { b.lo[a] = lo[a]; b.hi[a] = hi[a]; }
+    b.delta = dl;
+    b.count = cnt;
+    b.cost = W.cost[s];
+    b.left = W.left[lane];
+    b.right = W.right[lane];
+    const int32_t ch[2] = {W.left[lane], W.right[lane]};
+    for (int c = 0; c < 2; c++) {
+      if (ch[c] >= 0) nodes[ch[c]].parent = nd;
+      else leaf_parent[~ch[c]] = nd;
+    }
+  }
+}
+
 // Bottom-up: the second child to arrive restructures the treelet rooted at
 // its parent.  Everything below the root is final by then, and no other
-// thread touches it again; the root keeps its place (and parent).
-__global__ void k_treelets(const float* pos, const int32_t* sorted, const float* tdelta, int32_t n, BNode* nodes,
-                           int32_t* leaf_parent, int32_t* visits, int32_t* err) {
-  int32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= n) return;
-  int32_t cur = leaf_parent[k];
-  for (int32_t steps = 0; cur >= 0; steps++) {
-    if (steps >= n || cur >= n - 1) {  // a walk longer than the tree: corrupt links
+// warp touches it again; the root keeps its place (and parent).  A lane climbs
+// from each leaf; a node over two triangles is set by its lane, a larger one
+// by its lane's whole warp, one after the other.  (A thread per treelet kept
+// the subset costs and boxes in local memory: 300,000 triangles took 3.6 ms a
+// pass, 0.91 now; 1.18M triangles built in 32.4 ms, 9.9 now.)
+constexpr int kTreeletBlock = 128;
+__global__ void __launch_bounds__(kTreeletBlock)
+    k_treelets(const float* pos, const int32_t* sorted, const float* tdelta, int32_t n, BNode* nodes,
+               int32_t* leaf_parent, int32_t* visits, int32_t* err) {
+  __shared__ Treelet tl[kTreeletBlock / 32];
+  const int32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+  int32_t cur = k < n ? leaf_parent[k] : -1;
+  for (int32_t steps = 0;; steps++) {
+    if (cur >= 0 && (steps >= n || cur >= n - 1)) {  // a walk longer than the tree: corrupt links
       atomicOr(err, 1);
-      return;
+      cur = -1;
     }
-    __threadfence();
-    if (atomicAdd(&visits[cur], 1) == 0) return;
-    __threadfence();
-    BNode* R = nodes + cur;
-    // grow the treelet
-    int32_t T[kTreelet], I[kTreelet - 1];
-    int nt = 2, ni = 1;
-    T[0] = __ldcg(&R->left);
-    T[1] = __ldcg(&R->right);
-    I[0] = cur;
-    while (nt < kTreelet) {
-      int pick = -1;
-      float pa = -1.f;
-      for (int j = 0; j < nt; j++) {
-        if (T[j] < 0) continue;
-        const Sub sj = sub_of(nodes, pos, sorted, tdelta, T[j]);
-        const float a = area_of(sj.lo, sj.hi);
-        if (a > pa) { pa = a; pick = j; }
-      }
-      if (pick < 0) break;
-      const int32_t t = T[pick];
-      I[ni++] = t;
-      T[pick] = __ldcg(&nodes[t].left);
-      T[nt++] = __ldcg(&nodes[t].right);
-    }
-    if (nt >= 3) {
-      // least-cost topology over the treelet's leaves
-      float tlo[kTreelet][3], thi[kTreelet][3], tc[kTreelet];
-      for (int j = 0; j < nt; j++) {
-        const Sub sj = sub_of(nodes, pos, sorted, tdelta, T[j]);
-        for (int a = 0; a < 3; a++) { tlo[j][a] = sj.lo[a]; thi[j][a] = sj.hi[a]; }
-        tc[j] = sj.cost;
-      }
-      float cost[1 << kTreelet];
-      uint8_t part[1 << kTreelet];
-      const int full = (1 << nt) - 1;
-      for (int sset = 1; sset <= full; sset++) {
-        if ((sset & (sset - 1)) == 0) {
-          cost[sset] = tc[__ffs(sset) - 1];
-          continue;
-        }
-        float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
-        for (int j = 0; j < nt; j++)
-          if (sset >> j & 1)
-            for (int a = 0; a < 3; a++) { lo[a] = fminf(lo[a], tlo[j][a]); hi[a] = fmaxf(hi[a], thi[j][a]); }
-        const int low = sset & -sset, rest = sset ^ low;
-        float best = INFINITY;
-        int bp = low;
-        // partitions {low | q, rest \ q}, q a proper subset of rest
-        for (int q = (rest - 1) & rest;; q = (q - 1) & rest) {
-          const int pp = low | q;
-          const float c = cost[pp] + cost[sset ^ pp];
-          if (c < best) { best = c; bp = pp; }
-          if (q == 0) break;
-        }
-        cost[sset] = kSahNode * area_of(lo, hi) + best;
-        part[sset] = (uint8_t)bp;
-      }
-      // current cost of the treelet
-      const Sub l0 = sub_of(nodes, pos, sorted, tdelta, __ldcg(&R->left));
-      const Sub r0 = sub_of(nodes, pos, sorted, tdelta, __ldcg(&R->right));
-      float rlo[3], rhi[3];
-      for (int a = 0; a < 3; a++) { rlo[a] = fminf(l0.lo[a], r0.lo[a]); rhi[a] = fmaxf(l0.hi[a], r0.hi[a]); }
-      const float now = kSahNode * area_of(rlo, rhi) + l0.cost + r0.cost;
-      if (cost[full] < now * (1.0f - 1e-6f)) {
-        // rebuild with the internal nodes I (I[0] = the root), parents first
-        int32_t st_s[kTreelet], st_n[kTreelet];
-        int sp = 0, used = 1;
-        int32_t order[kTreelet - 1];
-        int no = 0;
-        st_s[sp] = full;
-        st_n[sp++] = cur;
-        while (sp > 0) {
-          const int sset = st_s[--sp];
-          const int32_t nd = st_n[sp];
-          order[no++] = nd;
-          const int sides[2] = {part[sset], sset ^ part[sset]};
-          int32_t ch[2];
-          for (int c = 0; c < 2; c++) {
-            if ((sides[c] & (sides[c] - 1)) == 0) {
-              ch[c] = T[__ffs(sides[c]) - 1];
-            } else {
-              ch[c] = I[used++];
-              st_s[sp] = sides[c];
-              st_n[sp++] = ch[c];
-            }
-            if (ch[c] >= 0) nodes[ch[c]].parent = nd;
-            else leaf_parent[~ch[c]] = nd;
-          }
-          nodes[nd].left = ch[0];
-          nodes[nd].right = ch[1];
-        }
-        // children before parents
-        for (int o = no - 1; o >= 0; o--) refit(nodes, pos, sorted, tdelta, order[o]);
+    bool whole = false;
+    if (cur >= 0) {
+      __threadfence();
+      if (atomicAdd(&visits[cur], 1) == 0) {
+        cur = -1;
       } else {
-        R->cost = now;
+        __threadfence();
+        whole = __ldcg(&nodes[cur].left) >= 0 || __ldcg(&nodes[cur].right) >= 0;
+        if (!whole) refit(nodes, pos, sorted, tdelta, cur);
       }
-    } else {
-      refit(nodes, pos, sorted, tdelta, cur);
     }
-    cur = __ldcg(&R->parent);
+    __syncwarp();
+    for (unsigned m = __ballot_sync(0xFFFFFFFFu, whole); m; m &= m - 1) {
+      restructure(pos, sorted, tdelta, nodes, leaf_parent, __shfl_sync(0xFFFFFFFFu, cur, __ffs(m) - 1),
+                  tl[threadIdx.x >> 5]);
+      __threadfence();
+      __syncwarp();
+    }
+    if (cur >= 0) cur = __ldcg(&nodes[cur].parent);
+    if (!__any_sync(0xFFFFFFFFu, cur >= 0)) return;
   }
 }
 
@@ -407,6 +505,10 @@ __global__ void k_node_ranges(BNode* nodes, const int32_t* pos_of, int32_t n_int
   nodes[i].last = ~c + nodes[i].count - 1;
 }
 
+// Levels launched before the host looks whether any is left: most scenes
+// need no more (300,000 triangles: 13), and a launch without items costs 2 us.
+constexpr int32_t kLevels = 16;
+
 struct Item {
   int32_t bnode;   // binary node to expand into a 4-wide node
   int32_t out;     // its 4-wide node index
@@ -436,12 +538,13 @@ __device__ __forceinline__ void child_info(const BNode* nodes, const float* pos,
   }
 }
 
-__global__ void k_collapse(const BNode* nodes, const float* pos, const int32_t* sorted, const float* tdelta,
-                           const Item* items, int32_t n_items, Item* next, int32_t* n_next, int32_t* n_out,
-                           float* out_nodes, int32_t max_leaf, int32_t* leaf_count) {
-  int32_t it = blockIdx.x * blockDim.x + threadIdx.x;
-  if (it >= n_items) return;
-  const Item I = items[it];
+// One level: items[0 .. *n_items) to 4-wide nodes, their internal children to
+// `next`.  The counts stay on the device, so that the levels are launched one
+// behind the other without a wait.
+__device__ __forceinline__ void collapse_item(const BNode* nodes, const float* pos, const int32_t* sorted,
+                                              const float* tdelta, const Item I, Item* next, int32_t* n_next,
+                                              int32_t* n_out, float* out_nodes, int32_t max_leaf,
+                                              int32_t* leaf_count) {
   int32_t ch[4];
   int32_t nc = 0;
   const BNode& root = nodes[I.bnode];
@@ -490,6 +593,13 @@ __global__ void k_collapse(const BNode* nodes, const float* pos, const int32_t* 
     nd[28 + s] = dl;
   }
 }
+__global__ void k_collapse(const BNode* nodes, const float* pos, const int32_t* sorted, const float* tdelta,
+                           const Item* items, const int32_t* n_items, Item* next, int32_t* n_next, int32_t* n_out,
+                           float* out_nodes, int32_t max_leaf, int32_t* leaf_count) {
+  const int32_t n = *n_items;
+  for (int32_t it = blockIdx.x * blockDim.x + threadIdx.x; it < n; it += gridDim.x * blockDim.x)
+    collapse_item(nodes, pos, sorted, tdelta, items[it], next, n_next, n_out, out_nodes, max_leaf, leaf_count);
+}
 
 // leaf-order triangle data (as scene.cpp lays it out on the host)
 __global__ void k_gather(const int32_t* sorted, int64_t n, const float* pos, const float* nrm, const float* uv,
@@ -520,18 +630,37 @@ __global__ void k_gather(const int32_t* sorted, int64_t n, const float* pos, con
   }
 }
 
+// Buffers of one build, cut from one allocation (`reserve`), further ones
+// only beyond it: an allocation and its release cost tens of microseconds
+// each, and a build takes about twenty buffers.
 struct Scratch {
   std::vector<void*> p;
+  char* at = nullptr;
+  size_t left = 0;
   ~Scratch() {
     for (void* q : p) cudaFree(q);
   }
-  er_status get(void** out, size_t bytes) {
-    cudaError_t e = cudaMalloc(out, std::max<size_t>(bytes, 16));
+  er_status reserve(size_t bytes) {
+    cudaError_t e = cudaMalloc((void**)&at, bytes);
     if (e != cudaSuccess) {
       cudaGetLastError();
+      at = nullptr;
+      left = 0;
       return fail(ER_ERR_OOM, "GPU BVH build buffers");
     }
-    p.push_back(*out);
+    p.push_back(at);
+    left = bytes;
+    return ER_OK;
+  }
+  er_status get(void** out, size_t bytes) {
+    bytes = (std::max<size_t>(bytes, 16) + 255) & ~(size_t)255;
+    if (bytes > left) {
+      er_status s = reserve(bytes);
+      if (s != ER_OK) return s;
+    }
+    *out = at;
+    at += bytes;
+    left -= bytes;
     return ER_OK;
   }
   template <typename T>
@@ -556,6 +685,12 @@ er_status build_bvh_gpu(er_scene* s, const er_scene_desc* d, int max_leaf, const
   max_leaf = std::min(std::max(max_leaf, 1), 8);
   Scratch X;
   er_status e;
+  const size_t nt = (size_t)std::max<int64_t>(T, 1);
+  // inputs, keys and links, binary and 4-wide nodes per triangle; the sort's
+  // space and the rounding of about twenty buffers
+  if ((e = X.reserve(nt * (9 * 4 * (d->tangents ? 3 : 2) + 6 * 4 + 4 * 4 + 28 + sizeof(BNode) + 16 + 128 +
+                           2 * sizeof(Item) + 16) + ((size_t)2 << 20))) != ER_OK)
+    return e;
   // raw triangle data on the device
   const float *pos, *nrm, *uv, *tan, *tsign;
   const int32_t *tobj, *omat;
@@ -619,7 +754,8 @@ er_status build_bvh_gpu(er_scene* s, const er_scene_desc* d, int max_leaf, const
     ER_CUDA(cudaMemsetAsync(terr, 0, 4, st));
     for (int pass = 0; pass < 3; pass++) {
       ER_CUDA(cudaMemsetAsync(visits, 0, (size_t)(n - 1) * 4, st));
-      k_treelets<<<(unsigned)((n + 127) / 128), 128, 0, st>>>(pos, sorted, tdelta, n, bn, leaf_parent, visits, terr);
+      k_treelets<<<(unsigned)((n + kTreeletBlock - 1) / kTreeletBlock), kTreeletBlock, 0, st>>>(pos, sorted, tdelta, n, bn,
+                                                                                                leaf_parent, visits, terr);
     }
     const unsigned gb = (unsigned)((n + 255) / 256);
     k_leaf_order<<<gb, 256, 0, st>>>(bn, leaf_parent, n, pos_of, terr);
@@ -637,12 +773,12 @@ er_status build_bvh_gpu(er_scene* s, const er_scene_desc* d, int max_leaf, const
   // top-down collapse into 4-wide nodes, one launch per level
   float* nodes4;
   Item *qa, *qb;
-  int32_t* counters;  // [0] next items [1] nodes [2] leaves
+  int32_t* counters;
   const size_t max_nodes = (size_t)std::max<int64_t>(T, 1);
   if ((e = X.get((void**)&nodes4, max_nodes * 128)) != ER_OK) return e;
   if ((e = X.get((void**)&qa, max_nodes * sizeof(Item))) != ER_OK) return e;
   if ((e = X.get((void**)&qb, max_nodes * sizeof(Item))) != ER_OK) return e;
-  if ((e = X.get((void**)&counters, 16)) != ER_OK) return e;
+  if ((e = X.get((void**)&counters, (kLevels + 3) * sizeof(int32_t))) != ER_OK) return e;
   int32_t node_count = 1, leaves = 0, depth = 1;
   if (n <= max_leaf) {
     // a root with a single leaf child (or, with no triangles, no child)
@@ -670,26 +806,28 @@ er_status build_bvh_gpu(er_scene* s, const er_scene_desc* d, int max_leaf, const
     }
     ER_CUDA(cudaMemcpyAsync(nodes4, root.data(), 128, cudaMemcpyHostToDevice, st));
   } else {
+    // counters: [0] nodes [1] leaves [2 + l] items of level l (kLevels at a time)
     Item first{0, 0};
     ER_CUDA(cudaMemcpyAsync(qa, &first, sizeof first, cudaMemcpyHostToDevice, st));
-    int32_t init[3] = {0, 1, 0};
-    ER_CUDA(cudaMemcpyAsync(counters, init, 12, cudaMemcpyHostToDevice, st));
-    int32_t n_items = 1;
+    int32_t c[kLevels + 3] = {1, 0, 1};
     depth = 0;
-    while (n_items > 0) {
-      depth++;
-      ER_CUDA(cudaMemsetAsync(counters, 0, 4, st));
-      k_collapse<<<(unsigned)((n_items + 127) / 128), 128, 0, st>>>(bn, pos, sorted, tdelta, qa, n_items, qb, counters,
-                                                                      counters + 1, nodes4, max_leaf, counters + 2);
+    while (c[2] > 0) {
+      ER_CUDA(cudaMemcpyAsync(counters, c, sizeof c, cudaMemcpyHostToDevice, st));
+      for (int32_t l = 0; l < kLevels; l++) {
+        k_collapse<<<(unsigned)(4 * s->num_sms), 128, 0, st>>>(bn, pos, sorted, tdelta, qa, counters + 2 + l, qb,
+                                                               counters + 3 + l, counters, nodes4, max_leaf,
+                                                               counters + 1);
+        std::swap(qa, qb);
+      }
       ER_CUDA(cudaGetLastError());
-      int32_t c[3];
-      ER_CUDA(cudaMemcpyAsync(c, counters, 12, cudaMemcpyDeviceToHost, st));
+      ER_CUDA(cudaMemcpyAsync(c, counters, sizeof c, cudaMemcpyDeviceToHost, st));
       ER_CUDA(cudaStreamSynchronize(st));
-      n_items = c[0];
-      node_count = c[1];
-      leaves = c[2];
-      std::swap(qa, qb);
+      for (int32_t l = 0; l < kLevels; l++) depth += c[2 + l] > 0;
+      c[2] = c[2 + kLevels];  // (the items left for a next round of levels)
+      for (int32_t l = 1; l <= kLevels; l++) c[2 + l] = 0;
     }
+    node_count = c[0];
+    leaves = c[1];
   }
   // outputs owned by the scene
   void *p_nodes, *p_tv, *p_tn, *p_tuv, *p_tt = nullptr;
