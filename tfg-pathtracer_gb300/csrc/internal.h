@@ -205,6 +205,11 @@ struct Film {
 
 struct Wave;  // wavefront buffers (render.cu)
 
+// er_trace_closest on host arrays, bytes of rays and hits (40 per ray): up to
+// kTracePinned in page-locked memory of the scene, up to kTraceKept in a
+// device block that stays with it.
+constexpr size_t kTracePinned = (size_t)1 << 19, kTraceKept = (size_t)1 << 24;
+
 // Per-wave constants of the sample loop (one job's slice of samples).
 struct WaveParams {
   int32_t W, H, npix, spp_wave, sample_base, max_depth;
@@ -300,8 +305,13 @@ struct er_scene {
   er::Wave* wave2 = nullptr;
   cudaStream_t stream2 = nullptr;
   // page-locked words read back by every render call without a blocking
-  // copy: the device error word at 0, the statistics counters at 64
+  // copy: the device error word at 0, the statistics counters at 64; from 128
+  // on kTracePinned bytes for the rays and hits of er_trace_closest
   unsigned char* h_pin = nullptr;
+  // device block of er_trace_closest on host arrays, kept between calls up to
+  // kTraceKept bytes
+  void* trace_dev = nullptr;
+  size_t trace_cap = 0;
   cudaEvent_t ev_fork = nullptr, ev_acc[2] = {nullptr, nullptr};
   uint32_t* err_word = nullptr;   // device error word (bounds / timeout)
   unsigned long long* d_stats = nullptr;  // device ray counters

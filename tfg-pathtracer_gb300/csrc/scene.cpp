@@ -234,7 +234,7 @@ extern "C" er_status er_scene_create(const er_scene_desc* d, const er_scene_opts
     }
     cudaEventCreate(&s->ev0);
     cudaEventCreate(&s->ev1);
-    ce = cudaHostAlloc((void**)&s->h_pin, 128, cudaHostAllocDefault);
+    ce = cudaHostAlloc((void**)&s->h_pin, 128 + kTracePinned, cudaHostAllocDefault);
     if (ce != cudaSuccess) return bail(cuda_fail(ce, "cudaHostAlloc"));
 
     // ---- BVH
@@ -460,6 +460,7 @@ extern "C" er_status er_scene_free(er_scene* s) {
     cudaFree(s->bw_rad);
     cudaFree(s->bw_b);
     cudaFree(s->kp_rad);
+    cudaFree(s->trace_dev);
     for (void* p : s->allocs) cudaFree(p);
     s->allocs.clear();
     for (cudaEvent_t e : s->ev_pool) cudaEventDestroy(e);
