@@ -222,6 +222,7 @@ er_status make_plan(er_batch* b, int64_t budget) {
       g.P.k0 = (uint32_t)J.seed;
       g.P.k1 = (uint32_t)(J.seed >> 32);
       g.P.flags = J.flags;
+      set_divisors(&g.P);
       segs.push_back(g);
       paths += (int64_t)sw * npix;
       w.n_acc += npix;

@@ -134,11 +134,35 @@ double shading_offset_bound(const er_scene_desc* d, int64_t i);
 
 // ----------------------------------------------------------- device scene --
 
+// Division of 0 <= a < 2^31 by an invariant d >= 1 as a multiplication
+// (T. Granlund, P. Montgomery, "Division by invariant integers using
+// multiplication", PLDI 1994): floor(a / d) = a * mul >> shift, two
+// instructions where the division by a variable takes about twenty.  A path's
+// pixel, the texel of an environment pick and the texture remainders took a
+// dozen divisions per vertex: 1080p at 16 samples 101.6 ms with them, 100.7
+// without; the 12-job batch 6.71 and 6.56.
+struct FastDiv {
+  uint32_t mul;
+  int32_t shift;
+#ifdef __CUDACC__
+  __host__ __device__
+#endif
+  int32_t operator()(int32_t a) const { return (int32_t)(((uint64_t)(uint32_t)a * mul) >> shift); }
+};
+inline FastDiv fast_div(int32_t d) {
+  if (d < 1) d = 1;
+  int32_t l = 0;
+  while (((int64_t)1 << l) < d) l++;
+  if (l == 0) return FastDiv{0x80000000u, 31};
+  return FastDiv{(uint32_t)((((uint64_t)1 << (31 + l)) / (uint32_t)d) + 1), 31 + l};
+}
+
 // Texture descriptor on the device (Texture.hpp:196-214).
 struct DevTex {
   int32_t w, h;
   int64_t offset;  // float4 texel offset into the texel pool
   float x_tile, y_tile, x_offset, y_offset;
+  FastDiv by_w;
 };
 
 // Camera with the per-ray trigonometry hoisted (kernel.cu:297-306).
@@ -215,7 +239,14 @@ struct WaveParams {
   int32_t W, H, npix, spp_wave, sample_base, max_depth;
   uint32_t k0, k1;
   uint32_t flags;
+  FastDiv by_w, by_tiles, by_group;  // W, whole tiles per row, paths per pixel group (set_divisors)
 };
+constexpr int kGroup = 2;  // log2 of the pixels per group of the path order (render.cu)
+inline void set_divisors(WaveParams* P) {
+  P->by_w = fast_div(P->W);
+  P->by_tiles = fast_div(P->W >> 3);
+  P->by_group = fast_div(P->spp_wave << kGroup);
+}
 
 // ------------------------------------------------------------------ batch --
 //

@@ -150,19 +150,27 @@ __device__ __forceinline__ f3 sample_adjoint(f3 L, float4 g4, uint32_t n) {
 // in one tile, so its primary rays and first hits are coherent), then the
 // columns and rows left over when the image does not divide into tiles.
 // pix = y * W + x.
-__device__ __forceinline__ int32_t tile_pixel(const WaveParams& P, int32_t q) {
+__device__ __forceinline__ void tile_pixel(const WaveParams& P, int32_t q, int32_t& x, int32_t& y) {
   const int32_t tw = P.W >> 3, th = P.H >> 2, rest = P.W & 7;
   if (q < tw * th * 32) {
-    const int32_t t = q >> 5, r = q & 31;
-    return (((t / tw) << 2) + (r >> 3)) * P.W + ((t % tw) << 3) + (r & 7);
+    const int32_t t = q >> 5, r = q & 31, ty = P.by_tiles(t);
+    x = ((t - ty * tw) << 3) + (r & 7);
+    y = (ty << 2) + (r >> 3);
+    return;
   }
   q -= tw * th * 32;
-  if (q < rest * th * 4) return (q / rest) * P.W + (tw << 3) + q % rest;
-  return th * 4 * P.W + q - rest * th * 4;
+  if (q < rest * th * 4) {
+    y = q / rest;
+    x = (tw << 3) + q - y * rest;
+    return;
+  }
+  q += th * 4 * tw * 8;  // (whole rows from here on)
+  y = P.by_w(q);
+  x = q - y * P.W;
 }
-__device__ __forceinline__ int32_t pixel_tile(const WaveParams& P, int32_t pix) {
-  const int32_t x = pix % P.W, y = pix / P.W, tw = P.W >> 3, th = P.H >> 2, rest = P.W & 7;
-  if (y >= th * 4) return pix;
+__device__ __forceinline__ int32_t pixel_tile(const WaveParams& P, int32_t x, int32_t y) {
+  const int32_t tw = P.W >> 3, th = P.H >> 2, rest = P.W & 7;
+  if (y >= th * 4) return y * P.W + x;
   if (x >= tw << 3) return tw * th * 32 + y * rest + x - (tw << 3);
   return (((y >> 2) * tw + (x >> 3)) << 5) + ((y & 3) << 3) + (x & 7);
 }
@@ -178,12 +186,11 @@ __device__ __forceinline__ int32_t pixel_tile(const WaveParams& P, int32_t pix) 
 // at 64 samples, forward and gradient, 46.1 -> 42.1 ms, of which 43.8 with
 // groups of 32 pixels; 641x479 at 9 samples 1.71 -> 1.63 ms; 1080p at 16
 // samples 110.6 -> 108.7 ms.
-constexpr int kGroup = 2;  // log2 of the pixels per group
-__device__ __forceinline__ void path_pixel(const WaveParams& P, int32_t local, int32_t& pix, int32_t& s) {
-  const int32_t per = P.spp_wave << kGroup, g = local / per, r = local - g * per;
-  const int32_t c = min(1 << kGroup, P.npix - (g << kGroup));
-  s = r / c;
-  pix = tile_pixel(P, (g << kGroup) + r - s * c);
+__device__ __forceinline__ void path_pixel(const WaveParams& P, int32_t local, int32_t& x, int32_t& y, int32_t& s) {
+  const int32_t g = P.by_group(local), r = local - g * (P.spp_wave << kGroup);
+  const int32_t c = P.npix - (g << kGroup);  // pixels left: the last group may have fewer
+  s = c >= 1 << kGroup ? r >> kGroup : r / c;
+  tile_pixel(P, (g << kGroup) + r - s * min(1 << kGroup, c), x, y);
 }
 // Index within its slice of sample s of the q-th pixel in tile order.
 __device__ __forceinline__ int32_t path_index(const WaveParams& P, int32_t q, int32_t s) {
@@ -201,9 +208,8 @@ __global__ void k_raygen(DevScene S, WaveView w, WaveParams P, int32_t n, BatchV
   if (p >= n) return;
   int32_t job;
   int32_t local = path_slice<BATCH>(B, p, P, job);
-  int32_t pix, s;
-  path_pixel(P, local, pix, s);
-  int32_t x = pix % P.W, y = pix / P.W;
+  int32_t x, y, s;
+  path_pixel(P, local, x, y, s);
   uint32_t idx = (uint32_t)out_index(P, x, y);
   uint32_t sample = (uint32_t)(P.sample_base + s);
   uint4 a = philox(make_uint4(idx, sample, 0u, 0u), P.k0, P.k1);
@@ -476,9 +482,9 @@ __global__ void __launch_bounds__(kShadeBlock, kShadeMinBlocks)
         if (bounce == 0 && w.aov)
           w.aovs[3 * (size_t)p] = w.aovs[3 * (size_t)p + 1] = w.aovs[3 * (size_t)p + 2] = make_float4(0, 0, 0, 0);
       } else {
-        int32_t pix, s;
-        path_pixel(P, local, pix, s);
-        uint32_t idx = (uint32_t)out_index(P, pix % P.W, pix / P.W);
+        int32_t x, y, s;
+        path_pixel(P, local, x, y, s);
+        uint32_t idx = (uint32_t)out_index(P, x, y);
         VertexShade V;
         shade_vertex<BATCH || GRAD>(S, P.flags, P.k0, P.k1, idx, (uint32_t)(P.sample_base + s), bounce, o, d, h.x, h.y, h.z,
                             slot, V);
@@ -583,7 +589,7 @@ __global__ void k_accumulate(WaveView w, WaveParams P, Film F, int32_t sw, Batch
 
 __device__ __forceinline__ void accumulate_pixel(const WaveView& w, const WaveParams& P, const Film& F, int32_t sw,
                                                  int32_t pix, int32_t path_base, uint32_t& bounce_sum) {
-  int32_t x = pix % P.W, y = pix / P.W;
+  const int32_t y = P.by_w(pix), x = pix - y * P.W;
   int32_t idx = out_index(P, x, y);
   uint32_t sa = F.samples[idx], pc = F.pathcount[idx];
   const bool fp64 = P.flags & ER_RENDER_ACCUM_FP64;
@@ -592,7 +598,7 @@ __device__ __forceinline__ void accumulate_pixel(const WaveView& w, const WavePa
   if (fp64) { s0 = F.sum[3 * (size_t)idx]; s1 = F.sum[3 * (size_t)idx + 1]; s2 = F.sum[3 * (size_t)idx + 2]; }
   float4 a[3];
   if (F.aov_on) for (int k = 0; k < 3; k++) a[k] = F.aov[k][idx];
-  const int32_t q = pixel_tile(P, pix);
+  const int32_t q = pixel_tile(P, x, y);
   for (int32_t s = 0; s < sw; s++) {
     int32_t p = path_base + path_index(P, q, s);
     float4 L = w.light[p];
@@ -649,9 +655,9 @@ __global__ void k_dump(WaveView w, WaveParams P, int32_t sw, int32_t s_off, floa
   if (p >= sw * P.npix) return;
   float4 L = w.light[p];
   resolve(w, p, L);
-  int32_t pix, s;
-  path_pixel(P, p, pix, s);
-  int64_t j = (int64_t)(s + s_off) * P.npix + out_index(P, pix % P.W, pix / P.W);
+  int32_t x, y, s;
+  path_pixel(P, p, x, y, s);
+  int64_t j = (int64_t)(s + s_off) * P.npix + out_index(P, x, y);
   rad[3 * j] = L.x; rad[3 * j + 1] = L.y; rad[3 * j + 2] = L.z;
   bnc[j] = (int32_t)(__float_as_uint(L.w) >> 8);
 }
@@ -898,6 +904,7 @@ er_status run(er_scene* s, const er_render_opts* o, float* dump_rad, int32_t* du
     cudaStream_t strm = alt ? s->stream2 : s->stream;
     int32_t cur = std::min(sw, o->spp - s0);
     P.spp_wave = cur;
+    set_divisors(&P);
     P.sample_base = o->sample_begin + s0;
     int32_t n = cur * npix;
     k_raygen<false><<<(n + 255) / 256, 256, 0, strm>>>(s->dev, w, P, n, NB, GradArgs{});
@@ -1047,6 +1054,7 @@ er_status render_backward_device(er_scene* s, const er_render_opts* o, const Gra
     cudaStream_t strm = alt ? s->stream2 : s->stream;
     const int32_t cur = std::min(sw, o->spp - s0);
     P.spp_wave = cur;
+    set_divisors(&P);
     P.sample_base = o->sample_begin + s0;
     const int32_t n = cur * npix;
     k_raygen<false, true><<<(n + 255) / 256, 256, 0, strm>>>(s->dev, w, P, n, NB, G);
@@ -1517,6 +1525,7 @@ extern "C" er_status er_render_noalloc(er_scene* s, const er_render_opts* o, flo
     for (int32_t s0 = 0; s0 < o->spp; s0 += sw) {
       int32_t cur = std::min(sw, o->spp - s0);
       P.spp_wave = cur;
+      set_divisors(&P);
       P.sample_base = o->sample_begin + s0;
       int32_t n = cur * (int32_t)npix;
       k_raygen<false><<<(n + 255) / 256, 256, 0, s->stream>>>(s->dev, w, P, n, NB, GradArgs{});  // also zeroes the queue counters

@@ -173,6 +173,7 @@ namespace {
 
 void pack_texels(const er_texture& t, std::vector<float4>& pool, DevTex* dt) {
   dt->w = t.width;
+  dt->by_w = fast_div(t.width);
   dt->h = t.height;
   dt->offset = (int64_t)pool.size();
   dt->x_tile = t.x_tile;

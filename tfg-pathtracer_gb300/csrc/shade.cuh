@@ -9,13 +9,19 @@
 
 namespace er {
 
+// x % n by the C remainder, without its division where x is in range already
+// (as it is unless a texture is tiled or offset).
+__device__ __forceinline__ int32_t rem_texel(int32_t x, int32_t n) { return (uint32_t)x < (uint32_t)n ? x : x % n; }
+__device__ __forceinline__ int32_t wrap_texel(int32_t x, int32_t n) {
+  x = rem_texel(x, n);
+  return x < 0 ? x + n : x;
+}
+
 // Texture.hpp:95-112 (nearest texel, tile/offset, C remainder; a negative
 // remainder is wrapped into range instead of reading outside the array).
 __device__ __forceinline__ f3 tex_coord(const DevScene& S, const DevTex& t, int32_t x, int32_t y) {
-  x = __float2int_rz(t.x_tile * ((float)x + t.x_offset * (float)t.w)) % t.w;
-  y = __float2int_rz(t.y_tile * ((float)y + t.y_offset * (float)t.h)) % t.h;
-  if (x < 0) x += t.w;
-  if (y < 0) y += t.h;
+  x = wrap_texel(__float2int_rz(t.x_tile * ((float)x + t.x_offset * (float)t.w)), t.w);
+  y = wrap_texel(__float2int_rz(t.y_tile * ((float)y + t.y_offset * (float)t.h)), t.h);
   float4 c = __ldg(S.texels + t.offset + (int64_t)y * t.w + x);
   return mk(c.x, c.y, c.z);
 }

@@ -12,10 +12,8 @@ namespace er {
 
 // Storage index of the texel tex_coord reads (Texture.hpp:95-112).
 __device__ __forceinline__ int64_t tex_index(const DevTex& t, int32_t x, int32_t y) {
-  x = __float2int_rz(t.x_tile * ((float)x + t.x_offset * (float)t.w)) % t.w;
-  y = __float2int_rz(t.y_tile * ((float)y + t.y_offset * (float)t.h)) % t.h;
-  if (x < 0) x += t.w;
-  if (y < 0) y += t.h;
+  x = wrap_texel(__float2int_rz(t.x_tile * ((float)x + t.x_offset * (float)t.w)), t.w);
+  y = wrap_texel(__float2int_rz(t.y_tile * ((float)y + t.y_offset * (float)t.h)), t.h);
   return (int64_t)y * t.w + x;
 }
 
@@ -49,10 +47,11 @@ __device__ __forceinline__ int32_t env_pick(const DevScene& S, uint32_t flags, u
 // kernel.cu:236-245: texel index -> pixel -> uv with the env's tile and
 // offset (Texture.hpp:177-193), limited to [0, 1] (Math.hpp:38-41).
 __device__ __forceinline__ void env_texel_uv(const DevTex& E, int32_t cnt, float& iu, float& iv) {
-  float nu = __fdiv_rn((float)(cnt % E.w), (float)E.w), nv = __fdiv_rn((float)(cnt / E.w), (float)E.h);
+  const int32_t row = E.by_w(cnt);
+  float nu = __fdiv_rn((float)(cnt - row * E.w), (float)E.w), nv = __fdiv_rn((float)row, (float)E.h);
   int32_t ix = __float2int_rz(nu * (float)E.w), iy = __float2int_rz(nv * (float)E.h);
-  ix = __float2int_rz(E.x_tile * ((float)ix - E.x_offset * (float)E.w)) % E.w;
-  iy = __float2int_rz(E.y_tile * ((float)iy - E.y_offset * (float)E.h)) % E.h;
+  ix = rem_texel(__float2int_rz(E.x_tile * ((float)ix - E.x_offset * (float)E.w)), E.w);
+  iy = rem_texel(__float2int_rz(E.y_tile * ((float)iy - E.y_offset * (float)E.h)), E.h);
   iu = __fdiv_rn((float)ix, (float)E.w);
   iv = __fdiv_rn((float)iy, (float)E.h);
   limit_uv(iu, iv);
