@@ -186,6 +186,7 @@ struct DevMaterial {
 
 struct DevScene {
   const float4* nodes;   // FP32 BVH4 (8 float4 per node)
+  cudaTextureObject_t node_tex;  // the same array as a linear texture, or 0 (node_texture)
   const uint4* qnodes;   // quantised BVH4 (4 uint4 per node) or null
   const float4* tri_v;   // 3 float4 per leaf slot: v0|desc id, v1|tie key, v2|material
   const float4* tri_n;   // 3 float4 per leaf slot: n0|tangent sign, n1, n2
@@ -372,6 +373,9 @@ namespace er {
 er_status dev_alloc(er_scene* s, void** p, size_t bytes);
 er_status upload(er_scene* s, void** p, const void* host, size_t bytes);
 DevCamera make_dev_camera(const er_camera& c);
+// A linear texture over n FP32 nodes for the traversal (scene.cpp); 0 where
+// plain loads serve better or a texture cannot hold them.
+er_status node_texture(const float4* nodes, int64_t n, int device, cudaTextureObject_t* out);
 void free_wave(er_scene* s);
 void free_film(er_scene* s);
 // Looks up (again) the device address of er_render_noalloc's scratch array

@@ -247,7 +247,7 @@ __device__ __forceinline__ void flush_counts(unsigned long long* stats, int k, c
 //
 // `phases` selects the phases (1 extension, 2 point-light, 4 env); a split
 // schedule runs them as three launches, the launch with phase 1 first.
-template <bool Q8, bool STATS, bool BATCH>
+template <int NODES, bool STATS, bool BATCH>
 __global__ void __launch_bounds__(kTravBlock, kTravMinBlocks)
     k_trace(DevScene S, WaveView w, int32_t b, uint32_t* err, BatchView B, uint32_t phases, int32_t min_width) {
   __shared__ int2 stk[kSmemStack * kTravBlock];
@@ -274,7 +274,7 @@ __global__ void __launch_bounds__(kTravBlock, kTravMinBlocks)
   const int64_t half = w.shadow_half;
   TravStats st{0, 0, 0}, ss{0, 0, 0};
   const int32_t width = rays_per_warp((int64_t)n_ext + n_pt + n_env, gridDim.x * (kTravBlock / 32), min_width);
-  persistent_traverse<kClosest, Q8, STATS>(
+  persistent_traverse<kClosest, NODES, STATS>(
       S, n_ext, &w.counts[kClaim], stk + threadIdx.x, st, err, width,
       [&](int32_t i, auto& tr) {
         float4 a = qo[i], d = qd[i];
@@ -287,7 +287,7 @@ __global__ void __launch_bounds__(kTravBlock, kTravMinBlocks)
       },
       [&](int32_t i, auto& tr) { hits[i] = make_float4(tr.t, tr.u, tr.v, __int_as_float(tr.slot)); });
   // point-light rays: shadow queue [half, half + n_pt)
-  persistent_traverse<kPoint, Q8, STATS>(
+  persistent_traverse<kPoint, NODES, STATS>(
       S, n_pt, &w.counts[kClaim + 1], stk + threadIdx.x, ss, err, width,
       [&](int32_t i, auto& tr) {
         float4 a = so[half + i], d = sd[half + i], p = spp[half + i];
@@ -300,7 +300,7 @@ __global__ void __launch_bounds__(kTravBlock, kTravMinBlocks)
       },
       [&](int32_t i, auto& tr) { vis[__float_as_int(so[half + i].w)] = tr.occluded ? 0 : 1; });
   // env rays: shadow queue [0, n_env)
-  persistent_traverse<kAny, Q8, STATS>(
+  persistent_traverse<kAny, NODES, STATS>(
       S, n_env, &w.counts[kClaim + 2], stk + threadIdx.x, ss, err, width,
       [&](int32_t i, auto& tr) {
         float4 a = so[i], d = sd[i];
@@ -700,6 +700,17 @@ int grid_for(K kernel, int block, int sms) {
   return blocks_per_sm((const void*)kernel, block) * sms;
 }
 
+// The traversal kernel for a scene's nodes (counted: plain or 8-bit only).
+using TraceFn = void (*)(DevScene, WaveView, int32_t, uint32_t*, BatchView, uint32_t, int32_t);
+template <bool BATCH>
+TraceFn trace_kernel(const DevScene& S, bool stats = false) {
+  const NodeKind kind = node_kind(S);
+  if (stats) return kind == kQ8Nodes ? k_trace<kQ8Nodes, true, BATCH> : k_trace<kPlainNodes, true, BATCH>;
+  return kind == kQ8Nodes    ? k_trace<kQ8Nodes, false, BATCH>
+         : kind == kTexNodes ? k_trace<kTexNodes, false, BATCH>
+                             : k_trace<kPlainNodes, false, BATCH>;
+}
+
 er_status alloc_w(Wave* w, void** p, size_t bytes) {
   cudaError_t e = cudaMalloc(p, std::max<size_t>(bytes, 16));
   if (e != cudaSuccess) {
@@ -853,7 +864,6 @@ er_status run(er_scene* s, const er_render_opts* o, float* dump_rad, int32_t* du
   P.W = W; P.H = H; P.npix = npix; P.max_depth = max_depth;
   P.k0 = (uint32_t)o->seed; P.k1 = (uint32_t)(o->seed >> 32);
   P.flags = o->flags;
-  const bool q8 = s->dev.use_q8;
   const bool count = o->flags & ER_RENDER_COUNT;
   const bool prof = o->flags & ER_RENDER_PROFILE;
   // Two waves in flight: wave k runs on stream k % 2 with its own buffers;
@@ -866,13 +876,10 @@ er_status run(er_scene* s, const er_render_opts* o, float* dump_rad, int32_t* du
     ER_CUDA(cudaEventRecord(s->ev_fork, s->stream));
     ER_CUDA(cudaStreamWaitEvent(s->stream2, s->ev_fork, 0));
   }
-  const int g_tr[4] = {grid_for(k_trace<false, false, false>, kTravBlock, s->num_sms),
-                       grid_for(k_trace<true, false, false>, kTravBlock, s->num_sms),
-                       grid_for(k_trace<false, true, false>, kTravBlock, s->num_sms),
-                       grid_for(k_trace<true, true, false>, kTravBlock, s->num_sms)};
+  const TraceFn k_tr = trace_kernel<false>(s->dev, count);
+  const int g_tr = grid_for(k_tr, kTravBlock, s->num_sms);
   const int g_shade = grid_for(k_shade<false>, 128, s->num_sms);
   const BatchView NB;
-  const int variant = (q8 ? 1 : 0) + (count ? 2 : 0);
   int64_t nl = 0;
   // Profiling: one event after every launch, attributed to its stage.
   s->ev_stage.clear();
@@ -913,12 +920,7 @@ er_status run(er_scene* s, const er_render_opts* o, float* dump_rad, int32_t* du
     // the extra trace(max_depth) finishes the last bounce's shadow rays.
     for (int32_t b = 0; b <= max_depth; b++) {
       uint32_t* err = s->err_word;
-      switch (variant) {
-        case 0: k_trace<false, false, false><<<g_tr[0], kTravBlock, 0, strm>>>(s->dev, w, b, err, NB, 7u, min_width); break;
-        case 1: k_trace<true, false, false><<<g_tr[1], kTravBlock, 0, strm>>>(s->dev, w, b, err, NB, 7u, min_width); break;
-        case 2: k_trace<false, true, false><<<g_tr[2], kTravBlock, 0, strm>>>(s->dev, w, b, err, NB, 7u, min_width); break;
-        default: k_trace<true, true, false><<<g_tr[3], kTravBlock, 0, strm>>>(s->dev, w, b, err, NB, 7u, min_width); break;
-      }
+      k_tr<<<g_tr, kTravBlock, 0, strm>>>(s->dev, w, b, err, NB, 7u, min_width);
       if ((st = mark(ER_STAGE_TRACE)) != ER_OK) return st;
       if (b == max_depth) break;
       if (eval) k_shade<false, false, true><<<g_shade, 128, 0, strm>>>(s->dev, w, P, b, NB, *eval);
@@ -1043,8 +1045,8 @@ er_status render_backward_device(er_scene* s, const er_render_opts* o, const Gra
   P.W = W; P.H = H; P.npix = npix; P.max_depth = max_depth;
   P.k0 = (uint32_t)o->seed; P.k1 = (uint32_t)(o->seed >> 32);
   P.flags = o->flags & ER_RENDER_ENV_ALIAS;
-  const int g_tr[2] = {grid_for(k_trace<false, false, false>, kTravBlock, s->num_sms),
-                       grid_for(k_trace<true, false, false>, kTravBlock, s->num_sms)};
+  const TraceFn k_tr = trace_kernel<false>(s->dev);
+  const int g_tr = grid_for(k_tr, kTravBlock, s->num_sms);
   const int g_sh = grid_for(k_shade<false, true>, 128, s->num_sms);
   const BatchView NB;
   int32_t k = 0;
@@ -1059,10 +1061,7 @@ er_status render_backward_device(er_scene* s, const er_render_opts* o, const Gra
     const int32_t n = cur * npix;
     k_raygen<false, true><<<(n + 255) / 256, 256, 0, strm>>>(s->dev, w, P, n, NB, G);
     for (int32_t b = 0; b <= max_depth; b++) {
-      if (s->dev.use_q8)
-        k_trace<true, false, false><<<g_tr[1], kTravBlock, 0, strm>>>(s->dev, w, b, s->err_word, NB, 7u, min_width);
-      else
-        k_trace<false, false, false><<<g_tr[0], kTravBlock, 0, strm>>>(s->dev, w, b, s->err_word, NB, 7u, min_width);
+      k_tr<<<g_tr, kTravBlock, 0, strm>>>(s->dev, w, b, s->err_word, NB, 7u, min_width);
       if (b == max_depth) break;
       k_shade<false, true><<<g_sh, 128, 0, strm>>>(s->dev, w, P, b, NB, G);
     }
@@ -1110,11 +1109,10 @@ er_status batch_launch(const DevScene& S, Wave* wv, const BatchSeg* d_segs, cons
                        const std::vector<BatchWave>& waves, const BatchSchedule& sch, int num_sms, uint32_t* err,
                        cudaStream_t stream, int64_t* launches, const BatchPair* pair) {
   // resident blocks per SM
-  const int occ_tr[2] = {blocks_per_sm((const void*)k_trace<false, false, true>, kTravBlock),
-                         blocks_per_sm((const void*)k_trace<true, false, true>, kTravBlock)};
+  const TraceFn k_tr = trace_kernel<true>(S);
+  const int occ_tr = blocks_per_sm((const void*)k_tr, kTravBlock);
   const int occ_sh = blocks_per_sm((const void*)k_shade<true>, 128);
-  const int q8 = S.use_q8 ? 1 : 0;
-  const int tb = sch.trace_blocks_per_sm > 0 ? std::min(sch.trace_blocks_per_sm, occ_tr[q8]) : occ_tr[q8];
+  const int tb = sch.trace_blocks_per_sm > 0 ? std::min(sch.trace_blocks_per_sm, occ_tr) : occ_tr;
   const int sb = sch.shade_blocks_per_sm > 0 ? std::min(sch.shade_blocks_per_sm, occ_sh) : occ_sh;
   const int g_tr = tb * num_sms, g_sh = sb * num_sms;
   if (launches) *launches = 0;
@@ -1134,8 +1132,7 @@ er_status batch_launch(const DevScene& S, Wave* wv, const BatchSeg* d_segs, cons
     const WaveView& w = wk->v;
     cudaStream_t strm = alt ? pair->s2 : stream;
     auto trace = [&](int32_t b, const BatchView& B, uint32_t phases) {
-      if (q8) k_trace<true, false, true><<<g_tr, kTravBlock, 0, strm>>>(S, w, b, err, B, phases, two ? 32 : kLoneWidth);
-      else k_trace<false, false, true><<<g_tr, kTravBlock, 0, strm>>>(S, w, b, err, B, phases, two ? 32 : kLoneWidth);
+      k_tr<<<g_tr, kTravBlock, 0, strm>>>(S, w, b, err, B, phases, two ? 32 : kLoneWidth);
       nl++;
     };
     if (bw.n_paths > wk->cap) return fail(ER_ERR_INVALID_ARG, "batch wave larger than its buffers");
@@ -1518,8 +1515,8 @@ extern "C" er_status er_render_noalloc(er_scene* s, const er_render_opts* o, flo
     P.W = W; P.H = H; P.npix = (int32_t)npix; P.max_depth = max_depth;
     P.k0 = (uint32_t)o->seed; P.k1 = (uint32_t)(o->seed >> 32);
     P.flags = 0;
-    const int g_tr = grid_for(k_trace<false, false, false>, kTravBlock, s->num_sms);
-    const int g_tr8 = grid_for(k_trace<true, false, false>, kTravBlock, s->num_sms);
+    const TraceFn k_tr = trace_kernel<false>(s->dev);
+    const int g_tr = grid_for(k_tr, kTravBlock, s->num_sms);
     const int g_sh = grid_for(k_shade<false>, 128, s->num_sms);
     const BatchView NB;
     for (int32_t s0 = 0; s0 < o->spp; s0 += sw) {
@@ -1530,10 +1527,7 @@ extern "C" er_status er_render_noalloc(er_scene* s, const er_render_opts* o, flo
       int32_t n = cur * (int32_t)npix;
       k_raygen<false><<<(n + 255) / 256, 256, 0, s->stream>>>(s->dev, w, P, n, NB, GradArgs{});  // also zeroes the queue counters
       for (int32_t b = 0; b <= max_depth; b++) {
-        if (s->dev.use_q8)
-          k_trace<true, false, false><<<g_tr8, kTravBlock, 0, s->stream>>>(s->dev, w, b, s->err_word, NB, 7u, kLoneWidth);
-        else
-          k_trace<false, false, false><<<g_tr, kTravBlock, 0, s->stream>>>(s->dev, w, b, s->err_word, NB, 7u, kLoneWidth);
+        k_tr<<<g_tr, kTravBlock, 0, s->stream>>>(s->dev, w, b, s->err_word, NB, 7u, kLoneWidth);
         if (b == max_depth) break;
         k_shade<false><<<g_sh, 128, 0, s->stream>>>(s->dev, w, P, b, NB, GradArgs{});
       }

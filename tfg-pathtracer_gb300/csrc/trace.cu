@@ -8,13 +8,13 @@
 namespace er {
 namespace {
 
-template <bool Q8, bool STATS>
+template <int NODES, bool STATS>
 __global__ void __launch_bounds__(kTravBlock, kTravMinBlocks)
     k_trace_rays(DevScene S, const float* __restrict__ rays, int32_t n, int normalize, int32_t* tri, float* dist,
                  float* uv, unsigned long long* stats, int32_t* counter, uint32_t* err) {
   __shared__ int2 stk[kSmemStack * kTravBlock];
   TravStats st{0, 0, 0};
-  persistent_traverse<kClosest, Q8, STATS>(
+  persistent_traverse<kClosest, NODES, STATS>(
       S, n, counter, stk + threadIdx.x, st, err,
       rays_per_warp(n, gridDim.x * (kTravBlock / 32), kLoneWidth),
       [&](int32_t i, auto& tr) {
@@ -39,15 +39,15 @@ __global__ void __launch_bounds__(kTravBlock, kTravMinBlocks)
   }
 }
 
-template <bool Q8, bool STATS>
+template <int NODES, bool STATS>
 void launch(er_scene* s, const float* rays, int64_t n, int normalize, int32_t* tri, float* dist, float* uv) {
-  const int grid = blocks_per_sm((const void*)k_trace_rays<Q8, STATS>, kTravBlock) * s->num_sms;
+  const int grid = blocks_per_sm((const void*)k_trace_rays<NODES, STATS>, kTravBlock) * s->num_sms;
   int64_t need = (n + kTravBlock / 32 * kLoneWidth - 1) / (kTravBlock / 32 * kLoneWidth);
   int g = (int)(need < grid ? need : grid);
   if (g < 1) g = 1;
   int32_t* counter = (int32_t*)((char*)s->err_word + 32);
   cudaMemsetAsync(counter, 0, sizeof(int32_t), s->stream);
-  k_trace_rays<Q8, STATS><<<g, kTravBlock, 0, s->stream>>>(s->dev, rays, (int32_t)n, normalize, tri, dist, uv,
+  k_trace_rays<NODES, STATS><<<g, kTravBlock, 0, s->stream>>>(s->dev, rays, (int32_t)n, normalize, tri, dist, uv,
                                                           s->d_stats, counter, s->err_word);
 }
 
@@ -111,12 +111,16 @@ extern "C" er_status er_trace_closest(er_scene* s, const float* rays, int64_t n,
     if (want_stats) cudaMemcpyAsync(s0, s->d_stats, sizeof s0, cudaMemcpyDeviceToHost, s->stream);
     cudaEventRecord(s->ev0, s->stream);
     int norm = (flags & ER_TRACE_NORMALIZED) ? 0 : 1;
-    if (s->dev.use_q8) {
-      if (want_stats) launch<true, true>(s, d_rays, n, norm, d_tri, d_dist, d_uv);
-      else launch<true, false>(s, d_rays, n, norm, d_tri, d_dist, d_uv);
+    const NodeKind kind = node_kind(s->dev);
+    if (kind == kQ8Nodes) {
+      if (want_stats) launch<kQ8Nodes, true>(s, d_rays, n, norm, d_tri, d_dist, d_uv);
+      else launch<kQ8Nodes, false>(s, d_rays, n, norm, d_tri, d_dist, d_uv);
+    } else if (want_stats) {
+      launch<kPlainNodes, true>(s, d_rays, n, norm, d_tri, d_dist, d_uv);
+    } else if (kind == kTexNodes) {
+      launch<kTexNodes, false>(s, d_rays, n, norm, d_tri, d_dist, d_uv);
     } else {
-      if (want_stats) launch<false, true>(s, d_rays, n, norm, d_tri, d_dist, d_uv);
-      else launch<false, false>(s, d_rays, n, norm, d_tri, d_dist, d_uv);
+      launch<kPlainNodes, false>(s, d_rays, n, norm, d_tri, d_dist, d_uv);
     }
     cudaEventRecord(s->ev1, s->stream);
     cudaError_t ce = cudaGetLastError();

@@ -25,6 +25,10 @@
 namespace er {
 
 enum TraceMode { kClosest = 0, kAny = 1, kPoint = 2 };
+// How nodes are read: FP32 nodes by plain loads, 8-bit nodes, FP32 nodes half
+// through the texture unit (node_texture, scene.cpp).
+enum NodeKind { kPlainNodes = 0, kQ8Nodes = 1, kTexNodes = 2 };
+inline NodeKind node_kind(const DevScene& S) { return S.use_q8 ? kQ8Nodes : S.node_tex ? kTexNodes : kPlainNodes; }
 
 #ifndef ER_TRAV_BLOCK
 #define ER_TRAV_BLOCK 128
@@ -143,8 +147,9 @@ __device__ __forceinline__ void planes4(float (&t)[4], float4 p, float a, float 
 //
 // Stack entries are (node or leaf reference, lower bound of the reference
 // distance of anything below it); leaves and internal nodes share the stack.
-template <int MODE, bool Q8, bool STATS>
+template <int MODE, int NODES, bool STATS>
 struct Traverser {
+  static constexpr bool Q8 = NODES == kQ8Nodes;
   f3 o, d, inv, pp;
   // Slab planes are evaluated as fma(plane, inv, bias): the near-plane bias
   // is lowered and the far-plane bias raised by a bound on the rounding
@@ -353,8 +358,23 @@ struct Traverser {
       dl = make_float4(dd, dd, dd, dd);
     } else {
       const float4* nd = S.nodes + 8 * (size_t)node;
-      const float4 nx = __ldg(nd + (sgn & 1u)), fx = __ldg(nd + 1 - (sgn & 1u));
-      const float4 ny = __ldg(nd + 2 + ((sgn >> 1) & 1u)), fy = __ldg(nd + 3 - ((sgn >> 1) & 1u));
+      // Eight scattered 16-byte loads per lane and node kept the load / store
+      // unit's data path 83 % busy, which bounded the kernel; four of them
+      // through the texture unit, which the kernel does not use otherwise,
+      // share the work (node_texture, scene.cpp).
+      float4 nx, fx, ny, fy;
+      if (NODES == kTexNodes) {
+        const int32_t e = 8 * node, sx = (int32_t)(sgn & 1u), sy = (int32_t)((sgn >> 1) & 1u);
+        nx = tex1Dfetch<float4>(S.node_tex, e + sx);
+        fx = tex1Dfetch<float4>(S.node_tex, e + 1 - sx);
+        ny = tex1Dfetch<float4>(S.node_tex, e + 2 + sy);
+        fy = tex1Dfetch<float4>(S.node_tex, e + 3 - sy);
+      } else {
+        nx = __ldg(nd + (sgn & 1u));
+        fx = __ldg(nd + 1 - (sgn & 1u));
+        ny = __ldg(nd + 2 + ((sgn >> 1) & 1u));
+        fy = __ldg(nd + 3 - ((sgn >> 1) & 1u));
+      }
       const float4 nz = __ldg(nd + 4 + ((sgn >> 2) & 1u)), fz = __ldg(nd + 5 - ((sgn >> 2) & 1u));
       float4 c4 = __ldg(nd + 6);
       ch = make_int4(__float_as_int(c4.x), __float_as_int(c4.y), __float_as_int(c4.z), __float_as_int(c4.w));
@@ -493,7 +513,7 @@ __device__ __forceinline__ int32_t rays_per_warp(int64_t n, int32_t n_warps, int
 // traversal.  Items are claimed in warp batches from *counter, which must be
 // zero at launch.  Only the first `width` lanes of a warp take items
 // (rays_per_warp).
-template <int MODE, bool Q8, bool STATS, typename Load, typename Store>
+template <int MODE, int NODES, bool STATS, typename Load, typename Store>
 __device__ __forceinline__ void persistent_traverse(const DevScene& S, int32_t n, int32_t* counter, int2* sstk,
                                                     TravStats& st, uint32_t* err, int32_t width, Load load,
                                                     Store store) {
@@ -501,7 +521,7 @@ __device__ __forceinline__ void persistent_traverse(const DevScene& S, int32_t n
   // launch of the same phase.
   if (n <= 0) return;
   int2 lstk[kLocalStack];
-  Traverser<MODE, Q8, STATS> tr;
+  Traverser<MODE, NODES, STATS> tr;
   const unsigned lane = threadIdx.x & 31u;
   int32_t item = (int32_t)lane < width ? -1 : n;  // -1: needs an item; >= n: queue exhausted
   const int32_t refill = min(kRefillThreshold, (width * 5) >> 3);
