@@ -370,12 +370,19 @@ constexpr int kShadeBlock = 128;
 // for the block to take 128 at a time.  Hits and escapes of a bounce after the
 // first lie mixed in the queue, and a warp that holds both runs the whole
 // vertex for its few hits and then the environment lookup for the others;
-// this leaves one mixed warp per block and group.  A block takes 4 x 128
-// items together when it has at least 8 such groups to do, so that the last
-// group costs little.  512x512 at 64 samples, forward and gradient: 36.1 ms,
-// with groups of 128 items 37.7, without 40.9 ms; groups of each warp alone
-// (no barrier, but the warps of a block drift apart in the code): 38.5.
-constexpr int kShadeRounds = 4;
+// this leaves one mixed warp per block and group.  512x512 at 64 samples,
+// forward and gradient: 36.1 ms with groups of 4 x 128 items, 37.7 with 128,
+// 40.9 ms without; groups of each warp alone (no barrier, but the warps of a
+// block drift apart in the code): 38.5.
+//
+// A block takes kShadeRounds x 128 items together when it has at least
+// kShadeLeast such groups to do, fewer otherwise: a large group leaves fewer
+// mixed warps, few of them an uneven end.  Gradient vertices cost so much more
+// than escapes that the larger and fewer groups pay (4 x 128 of at least 8:
+// 33.3 ms for the workload above, of at least 2: 32.9, 8 x 128 of 2: 32.6,
+// 16 x 128: 32.9); in a batch most rays escape (12 jobs: 6.51 ms with at least
+// 8, 6.43 with 2); a single wave at 1080p loses 1 % with 2 (7.38 to 7.46 ms).
+template <int32_t kShadeRounds>
 __device__ __forceinline__ void hits_first(const float4* hits, int32_t base, int32_t n, int32_t rounds,
                                            int32_t* s_hits, int32_t* s_item) {
   constexpr int32_t kWarps = kShadeBlock / 32;
@@ -417,12 +424,13 @@ __global__ void __launch_bounds__(kShadeBlock, kShadeMinBlocks)
     w.counts[kClaim + 1] = 0;
     w.counts[kClaim + 2] = 0;
   }
+  constexpr int32_t kShadeRounds = GRAD ? 8 : 4, kShadeLeast = GRAD || BATCH ? 2 : 8;
   __shared__ int32_t s_item[kShadeRounds * kShadeBlock];
   __shared__ int32_t s_hits[kShadeRounds * kShadeBlock / 32];
-  const int32_t rounds = min(kShadeRounds, max(1, n / (8 * kShadeBlock * (int32_t)gridDim.x)));
+  const int32_t rounds = min(kShadeRounds, max(1, n / (kShadeLeast * kShadeBlock * (int32_t)gridDim.x)));
   const int32_t per = rounds * kShadeBlock;
   for (int32_t base = blockIdx.x * per, round = 0; base < n;) {
-    if (round == 0) hits_first(w.hits, base, n, rounds, s_hits, s_item);
+    if (round == 0) hits_first<kShadeRounds>(w.hits, base, n, rounds, s_hits, s_item);
     const int32_t i = s_item[round * kShadeBlock + threadIdx.x];
     if (++round == rounds) {
       round = 0;
