@@ -149,8 +149,9 @@ struct FastDiv {
 #endif
   int32_t operator()(int32_t a) const { return (int32_t)(((uint64_t)(uint32_t)a * mul) >> shift); }
 };
-inline FastDiv fast_div(int32_t d) {
+inline FastDiv fast_div(int64_t d) {
   if (d < 1) d = 1;
+  if (d > INT32_MAX) return FastDiv{0, 0};  // above every dividend
   int32_t l = 0;
   while (((int64_t)1 << l) < d) l++;
   if (l == 0) return FastDiv{0x80000000u, 31};
@@ -246,7 +247,7 @@ constexpr int kGroup = 2;  // log2 of the pixels per group of the path order (re
 inline void set_divisors(WaveParams* P) {
   P->by_w = fast_div(P->W);
   P->by_tiles = fast_div(P->W >> 3);
-  P->by_group = fast_div(P->spp_wave << kGroup);
+  P->by_group = fast_div((int64_t)P->spp_wave << kGroup);
 }
 
 // ------------------------------------------------------------------ batch --

@@ -175,6 +175,10 @@ __device__ __forceinline__ int32_t pixel_tile(const WaveParams& P, int32_t x, in
   return (((y >> 2) * tw + (x >> 3)) << 5) + ((y & 3) << 3) + (x & 7);
 }
 
+// Paths of a whole group of pixels.  From 2^29 samples per pixel on this does
+// not fit an int, later not 32 bits; a wave is then one group, the 0th.
+__device__ __forceinline__ uint32_t group_paths(const WaveParams& P) { return (uint32_t)P.spp_wave << kGroup; }
+
 // Path order of a slice: groups of four pixels in tile order, all samples
 // of a group together (the last group may have fewer pixels).  A warp of a
 // many-sample wave thus starts in one or two pixels, so its rays, hits,
@@ -187,7 +191,7 @@ __device__ __forceinline__ int32_t pixel_tile(const WaveParams& P, int32_t x, in
 // groups of 32 pixels; 641x479 at 9 samples 1.71 -> 1.63 ms; 1080p at 16
 // samples 110.6 -> 108.7 ms.
 __device__ __forceinline__ void path_pixel(const WaveParams& P, int32_t local, int32_t& x, int32_t& y, int32_t& s) {
-  const int32_t g = P.by_group(local), r = local - g * (P.spp_wave << kGroup);
+  const int32_t g = P.by_group(local), r = local - (int32_t)(g * group_paths(P));
   const int32_t c = P.npix - (g << kGroup);  // pixels left: the last group may have fewer
   s = c >= 1 << kGroup ? r >> kGroup : r / c;
   tile_pixel(P, (g << kGroup) + r - s * min(1 << kGroup, c), x, y);
@@ -195,7 +199,7 @@ __device__ __forceinline__ void path_pixel(const WaveParams& P, int32_t local, i
 // Index within its slice of sample s of the q-th pixel in tile order.
 __device__ __forceinline__ int32_t path_index(const WaveParams& P, int32_t q, int32_t s) {
   const int32_t g = q >> kGroup, c = min(1 << kGroup, P.npix - (g << kGroup));
-  return g * (P.spp_wave << kGroup) + s * c + (q & ((1 << kGroup) - 1));
+  return (int32_t)(g * group_paths(P)) + s * c + (q & ((1 << kGroup) - 1));
 }
 
 template <bool BATCH, bool GRAD = false>
