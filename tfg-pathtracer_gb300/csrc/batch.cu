@@ -490,8 +490,7 @@ extern "C" er_status er_batch_create(er_scene* const* scenes, int32_t n_scenes, 
     DevScene& M = b->dev;
     M = b->scenes[0]->dev;  // per-job parts (env, lights, camera) come from the job table
     M.nodes = (const float4*)p_nodes;
-    M.node_tex = 0;  // (the scene's own covers its own nodes)
-    if ((st = node_texture(M.nodes, nodes, device, &M.node_tex)) != ER_OK) return bail(st);
+    M.node_tex = node_texture(M.nodes, nodes, device);  // (the scene's own covers its own nodes)
     M.qnodes = (const uint4*)p_q;
     M.tri_v = (const float4*)p_tv;
     M.tri_n = (const float4*)p_tn;

@@ -375,8 +375,8 @@ er_status dev_alloc(er_scene* s, void** p, size_t bytes);
 er_status upload(er_scene* s, void** p, const void* host, size_t bytes);
 DevCamera make_dev_camera(const er_camera& c);
 // A linear texture over n FP32 nodes for the traversal (scene.cpp); 0 where
-// plain loads serve better or a texture cannot hold them.
-er_status node_texture(const float4* nodes, int64_t n, int device, cudaTextureObject_t* out);
+// plain loads serve better, a texture cannot hold them or none is to be had.
+cudaTextureObject_t node_texture(const float4* nodes, int64_t n, int device);
 void free_wave(er_scene* s);
 void free_film(er_scene* s);
 // Looks up (again) the device address of er_render_noalloc's scratch array

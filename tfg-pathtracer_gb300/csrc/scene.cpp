@@ -72,11 +72,14 @@ DevCamera make_dev_camera(const er_camera& c) {
 // texture: 73.9 ms of tracing; four 71.0, six 72.3; four and the triangles
 // 71.8; all and the triangles 77.5.)
 constexpr int64_t kTexLeast = 4096;
-er_status node_texture(const float4* nodes, int64_t n, int device, cudaTextureObject_t* out) {
-  *out = 0;
+cudaTextureObject_t node_texture(const float4* nodes, int64_t n, int device) {
   int most = 0;
-  ER_CUDA(cudaDeviceGetAttribute(&most, cudaDevAttrMaxTexture1DLinearWidth, device));
-  if (n < kTexLeast || 8 * n > (int64_t)most) return ER_OK;
+  if (n < kTexLeast) return 0;
+  if (cudaDeviceGetAttribute(&most, cudaDevAttrMaxTexture1DLinearWidth, device) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  if (8 * n > (int64_t)most) return 0;
   cudaResourceDesc r{};
   r.resType = cudaResourceTypeLinear;
   r.res.linear.devPtr = const_cast<float4*>(nodes);
@@ -84,8 +87,12 @@ er_status node_texture(const float4* nodes, int64_t n, int device, cudaTextureOb
   r.res.linear.sizeInBytes = (size_t)n * 128;
   cudaTextureDesc t{};
   t.readMode = cudaReadModeElementType;
-  ER_CUDA(cudaCreateTextureObject(out, &r, &t, nullptr));
-  return ER_OK;
+  cudaTextureObject_t tex = 0;
+  if (cudaCreateTextureObject(&tex, &r, &t, nullptr) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  return tex;
 }
 
 er_status check_device_error(er_scene* s) {
@@ -398,7 +405,7 @@ extern "C" er_status er_scene_create(const er_scene_desc* d, const er_scene_opts
 
     DevScene& S = s->dev;
     S.nodes = (const float4*)p_nodes;
-    if ((st = node_texture(S.nodes, br.node_count, s->device, &S.node_tex)) != ER_OK) return bail(st);
+    S.node_tex = node_texture(S.nodes, br.node_count, s->device);
     S.qnodes = (const uint4*)p_q;
     S.tri_v = (const float4*)p_tv;
     S.tri_n = (const float4*)p_tn;
