@@ -233,8 +233,11 @@ struct Wave;  // wavefront buffers (render.cu)
 
 // er_trace_closest on host arrays, bytes of rays and hits (40 per ray): up to
 // kTracePinned in page-locked memory of the scene, up to kTraceKept in a
-// device block that stays with it.
+// device block that stays with it.  All scenes of a process together hold at
+// most kTracePinnedAll page-locked bytes for rays: those created beyond that,
+// or where the system has none to give, use the device block for few rays too.
 constexpr size_t kTracePinned = (size_t)1 << 19, kTraceKept = (size_t)1 << 24;
+constexpr size_t kTracePinnedAll = (size_t)1 << 24;
 
 // Per-wave constants of the sample loop (one job's slice of samples).
 struct WaveParams {
@@ -338,9 +341,11 @@ struct er_scene {
   er::Wave* wave2 = nullptr;
   cudaStream_t stream2 = nullptr;
   // page-locked words read back by every render call without a blocking
-  // copy: the device error word at 0, the statistics counters at 64; from 128
-  // on kTracePinned bytes for the rays and hits of er_trace_closest
+  // copy: the device error word at 0, the statistics counters at 64; with
+  // pin_rays from 128 on kTracePinned bytes for the rays and hits of
+  // er_trace_closest
   unsigned char* h_pin = nullptr;
+  bool pin_rays = false;
   // device block of er_trace_closest on host arrays, kept between calls up to
   // kTraceKept bytes
   void* trace_dev = nullptr;

@@ -5,6 +5,7 @@
 // on the host once (leaf order for the triangle data) and uploaded into
 // allocations owned by the handle.
 #include <algorithm>
+#include <atomic>
 #include <chrono>
 #include <cmath>
 #include <cstring>
@@ -94,6 +95,25 @@ cudaTextureObject_t node_texture(const float4* nodes, int64_t n, int device) {
   }
   return tex;
 }
+
+namespace {
+
+std::atomic<size_t> g_pinned_rays{0};  // of all scenes of the process
+
+// s->h_pin.  The space for rays is made with the scene: a first call of 4,099
+// rays takes 119 us then, 250 if it has to page-lock the space itself.
+er_status alloc_pinned(er_scene* s) {
+  s->pin_rays = g_pinned_rays.fetch_add(kTracePinned) + kTracePinned <= kTracePinnedAll &&
+                cudaHostAlloc((void**)&s->h_pin, 128 + kTracePinned, cudaHostAllocDefault) == cudaSuccess;
+  if (s->pin_rays) return ER_OK;
+  cudaGetLastError();
+  g_pinned_rays -= kTracePinned;
+  s->h_pin = nullptr;
+  ER_CUDA(cudaHostAlloc((void**)&s->h_pin, 128, cudaHostAllocDefault));
+  return ER_OK;
+}
+
+}  // namespace
 
 er_status check_device_error(er_scene* s) {
   uint32_t w = 0;
@@ -267,8 +287,7 @@ extern "C" er_status er_scene_create(const er_scene_desc* d, const er_scene_opts
     }
     cudaEventCreate(&s->ev0);
     cudaEventCreate(&s->ev1);
-    ce = cudaHostAlloc((void**)&s->h_pin, 128 + kTracePinned, cudaHostAllocDefault);
-    if (ce != cudaSuccess) return bail(cuda_fail(ce, "cudaHostAlloc"));
+    if ((st = alloc_pinned(s)) != ER_OK) return bail(st);
 
     // ---- BVH
     const bool gpu_build = o.builder == ER_BUILDER_GPU;
@@ -502,6 +521,7 @@ extern "C" er_status er_scene_free(er_scene* s) {
     if (s->ev0) cudaEventDestroy(s->ev0);
     if (s->ev1) cudaEventDestroy(s->ev1);
     if (s->h_pin) cudaFreeHost(s->h_pin);
+    if (s->pin_rays) g_pinned_rays -= kTracePinned;
     cudaFree(s->snap_beauty);
     cudaFree(s->snap_samples);
     if (s->snap_event) cudaEventDestroy(s->snap_event);

@@ -69,14 +69,14 @@ extern "C" er_status er_trace_closest(er_scene* s, const float* rays, int64_t n,
     int32_t* d_tri = tri_id;
     float *d_dist = dist, *d_uv = uv;
     // Host arrays.  Few rays (kTracePinned) are copied into page-locked memory
-    // of the scene, which the kernel reads and writes in place: no transfers
-    // and nothing to allocate.  More go through one device block, rays first;
-    // up to kTraceKept it stays with the scene for its next call.  4,099 rays
-    // take 61 us a call; with an allocation per array, a transfer each and two
-    // waits they took 114.
+    // of the scene, where it has it, which the kernel reads and writes in
+    // place: no transfers and nothing to allocate.  Others go through one
+    // device block, rays first; up to kTraceKept it stays with the scene for
+    // its next call.  4,099 rays take 58 us a call, 88 through the block; with
+    // an allocation per array, a transfer each and two waits they took 114.
     const size_t n4 = ((size_t)n * 4 + 255) & ~(size_t)255;
     const size_t in_bytes = 6 * n4, bytes = in_bytes + (1 + (dist ? 1 : 0) + (uv ? 2 : 0)) * n4;
-    const bool pinned = !dev && bytes <= kTracePinned;
+    const bool pinned = !dev && s->pin_rays && bytes <= kTracePinned;
     char* block = (char*)s->h_pin + 128;
     void* own = nullptr;  // a block of this call alone
     if (!dev) {
