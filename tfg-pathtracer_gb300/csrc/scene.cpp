@@ -474,7 +474,7 @@ extern "C" er_status er_scene_info_get(const er_scene* s, er_scene_info* out) {
   return guarded("er_scene_info_get", [&]() -> er_status {
     if (!s || !out) return fail(ER_ERR_INVALID_ARG, "NULL argument");
     *out = s->info;
-    out->device_bytes = s->device_bytes;
+    out->device_bytes = s->device_bytes + (int64_t)s->trace_cap;
     return ER_OK;
   });
 }
