@@ -699,8 +699,9 @@ extern "C" er_status er_batch_free(er_batch* b) {
     cudaSetDevice(b->device);
     if (b->stream) cudaStreamSynchronize(b->stream);
     drop_graph(b);
-    if (b->dev.node_tex) cudaDestroyTextureObject(b->dev.node_tex);
+    // (a render that failed part-way may have left launches on it)
     if (b->pair.s2) cudaStreamSynchronize(b->pair.s2);
+    if (b->dev.node_tex) cudaDestroyTextureObject(b->dev.node_tex);
     wave_destroy(b->wave);
     wave_destroy(b->pair.w2);
     for (void* p : b->allocs) cudaFree(p);
