@@ -168,8 +168,11 @@ __global__ void k_post(const float4* in, float4* out, uchar4* ldr, PostParams P)
 // ACES, sRGB, 8-bit output, per call: half-width 4 136 us, 24 1.95 ms; 2.51
 // and 5.59 ms as three passes that read every tap from global memory, with
 // the double expressions and an allocation per buffer and call.  320x240 with
-// half-width 4: 33 and 310 us.  The weights come as a kernel parameter.
-constexpr int kTileBlur = 24;  // 80 x 80 pixels of 16 bytes: two blocks per SM
+// half-width 4: 33 and 310 us.  The weights come as a kernel parameter.  Two
+// blocks share an SM up to half-width 23 (78 x 78 pixels and the weights, 115
+// KB), one has it from 24 on (122 KB): 1.37 and 1.95 ms, against 3.25 and
+// 3.48 with the passes for wider blurs.
+constexpr int kTileBlur = 24;
 struct BlurWeights {
   float w[(2 * kTileBlur + 1) * (2 * kTileBlur + 1)];
   float one;  // 1 (tap)

@@ -361,11 +361,10 @@ __device__ __forceinline__ void grad_prev_vertex(const WaveView& w, const GradAr
 #endif
 // Resident 128-thread shade blocks per SM the register budgets are sized
 // for (72 registers).  The kernels wait on dependent loads (texture, material,
-// env lookups, atomics), so occupancy pays for some spilling.  Forward:
-// unbounded 117 registers at 4 blocks, 10 % longer stage on the 1080p scene;
-// 6 and 8 blocks 27.2 ms against 24.6 for 16 samples.  Gradient: 512x512 at
-// 64 samples, forward and gradient, 37.7 ms at 7 blocks, 37.8 at 6, 38.4 at
-// 10, 38.8 at 12.
+// env lookups, atomics), so occupancy pays for some spilling.  Blocks 4, 5, 6,
+// 7, 8, 10, 12, ms: the shade stage of 16 samples at 1080p 21.4, 20.3, 20.0,
+// 20.4, 21.0, 22.4, 24.7; 512x512 at 64 samples, forward and gradient, 32.7,
+// 32.9, 32.7, 32.6, 32.7, 33.2, 34.0.
 constexpr int kShadeMinBlocks = ER_SHADE_MIN_BLOCKS;
 constexpr int kShadeBlock = 128;
 
